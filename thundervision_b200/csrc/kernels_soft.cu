@@ -26,6 +26,8 @@
 #include <math_constants.h>
 
 #include <cstdint>
+#include <initializer_list>
+#include <type_traits>
 
 #include "tdv_internal.hpp"
 
@@ -56,6 +58,68 @@ __device__ __forceinline__ T warp_minv(T v) {
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) v = fmin(v, shfl_xor(v, s));
     return v;
+}
+// float: one reduction instruction instead of five shuffles and minima on the
+// recurrence's dependency chain (NaN ignored, as fmin does)
+template <>
+__device__ __forceinline__ float warp_minv<float>(float v) {
+    float r;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// A lane's NPL consecutive values at p.  VEC: D is a multiple of NPL and of
+// 16 bytes and every volume is 16-byte aligned, so a lane's values are all
+// inside the pixel's run or all outside (`in`) and move as one or more
+// vectors of up to 16 bytes; otherwise one predicated scalar per value.
+template <typename T, int NPL>
+constexpr int vec_elems() {
+    return NPL * (int)sizeof(T) >= 16 ? 16 / (int)sizeof(T) : NPL;
+}
+template <typename T, int NPL, bool VEC>
+__device__ __forceinline__ void load_run(const T* p, int d0, int D, T fill, T* v) {
+    if constexpr (VEC) {
+        constexpr int E = vec_elems<T, NPL>();
+        struct alignas(E * sizeof(T)) Chunk {
+            T e[E];
+        };
+        if (d0 < D) {
+#pragma unroll
+            for (int i = 0; i < NPL / E; i++) {
+                const Chunk c = *reinterpret_cast<const Chunk*>(p + i * E);
+#pragma unroll
+                for (int j = 0; j < E; j++) v[i * E + j] = c.e[j];
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < NPL; j++) v[j] = fill;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < NPL; j++) v[j] = d0 + j < D ? p[j] : fill;
+    }
+}
+template <typename T, int NPL, bool VEC>
+__device__ __forceinline__ void store_run(T* p, int d0, int D, const T* v) {
+    if constexpr (VEC) {
+        constexpr int E = vec_elems<T, NPL>();
+        struct alignas(E * sizeof(T)) Chunk {
+            T e[E];
+        };
+        if (d0 < D) {
+#pragma unroll
+            for (int i = 0; i < NPL / E; i++) {
+                Chunk c;
+#pragma unroll
+                for (int j = 0; j < E; j++) c.e[j] = v[i * E + j];
+                *reinterpret_cast<Chunk*>(p + i * E) = c;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < NPL; j++)
+            if (d0 + j < D) p[j] = v[j];
+    }
 }
 
 __device__ __forceinline__ void walk_geom(int i, int dx, int dy, int W, int H, int& sx, int& sy,
@@ -158,18 +222,22 @@ __device__ __forceinline__ void soft_step(const T* L, T m, const T* c, T p1, T p
     }
 }
 
-// lowest-index minimum of a warp's values
+// minimum of a warp's values
 template <typename T, int NPL>
-__device__ __forceinline__ void warp_argmin(const T* L, int d0, T& m, int& k) {
+__device__ __forceinline__ T run_min(const T* L) {
     T lm = L[0];
 #pragma unroll
     for (int j = 1; j < NPL; j++) lm = fmin(lm, L[j]);
-    m = warp_minv(lm);
+    return warp_minv(lm);
+}
+// lowest index that holds the minimum m
+template <typename T, int NPL>
+__device__ __forceinline__ int run_argmin(const T* L, T m, int d0) {
     int kk = 0x7FFFFFFF;
 #pragma unroll
     for (int j = NPL - 1; j >= 0; j--)
         if (L[j] == m) kk = d0 + j;
-    k = (int)__reduce_min_sync(FULLM, (uint32_t)kk);
+    return (int)__reduce_min_sync(FULLM, (uint32_t)kk);
 }
 
 template <typename T, int NPL>
@@ -187,8 +255,23 @@ __device__ __forceinline__ uint32_t load_codes(const uint8_t* src) {
     return *(const uint32_t*)src;
 }
 
+// Steps of C (forward, segment recomputation) or dS (adjoint) a walk keeps in
+// flight: a walk's next load address does not depend on the recurrence, so the
+// loads run ahead of it in a register ring.
+template <typename T, int NPL>
+constexpr int run_ahead() {
+    return NPL * (int)sizeof(T) <= 16 ? 4 : 2;
+}
+
 // REC: 0 = no tape (inference), 1 = codes, 2 = checkpoints.
-template <typename T, int NPL, int REC>
+//
+// What bounds it: at 960x540, D = 128 the 8 directions write 2.1 GB of L and
+// read C 8 times (1.2 GB from DRAM, the rest from L2), 0.51 ms at the measured
+// copy bandwidth.  One load of C per step issued when it is needed, as four
+// scalars per lane with 16-byte strides, took 0.95 ms (every step waiting for
+// its own load, 514 M warp instructions); with the load ring, whole-vector
+// accesses and the one-instruction warp minimum it takes 0.67 ms.
+template <typename T, int NPL, int REC, bool VEC>
 __global__ void __launch_bounds__(128) soft_fwd_pass(SoftK<T> k, int nd) {
     const int lane = threadIdx.x & 31;
     int dir, wblk;
@@ -204,73 +287,92 @@ __global__ void __launch_bounds__(128) soft_fwd_pass(SoftK<T> k, int nd) {
     const T inf = inf_v<T>();
     const size_t npix = (size_t)k.W * k.H;
     constexpr int CB = CodeWord<NPL>::kBytes;
-    uint8_t* codes = k.codes ? k.codes + (size_t)dir * npix * 32 * CB : nullptr;
-    uint16_t* kst = k.kstar ? k.kstar + (size_t)dir * npix : nullptr;
-    T* ck = (REC == 2) ? k.ckpt + (size_t)k.ckpt_off[(size_t)dir * (k.W + k.H) + w] * D : nullptr;
-    T* Lout = k.part + (size_t)dir * npix * D;
+    constexpr int K = run_ahead<T, NPL>();
+    const long long pstep = (long long)dy * k.W + dx;  // pixels from one step to the next
+    const long long p0 = (long long)sy * k.W + sx;
+    uint8_t* codes = REC == 1 ? k.codes + ((size_t)dir * npix + p0) * 32 * CB + lane * CB : nullptr;
+    uint16_t* kst = REC == 1 ? k.kstar + (size_t)dir * npix + p0 : nullptr;
+    T* ck = REC == 2 ? k.ckpt + (size_t)k.ckpt_off[(size_t)dir * (k.W + k.H) + w] * D + d0 : nullptr;
+    const T* Cq = k.C + p0 * D + d0;
+    T* Lq = k.part + ((size_t)dir * npix + p0) * D + d0;
+    const long long vstep = pstep * D;
 
-    T L[NPL], c[NPL], Ln[NPL];
-    int x = sx, y = sy;
-    size_t p = (size_t)y * k.W + x;
+    T L[NPL];
+    load_run<T, NPL, VEC>(Cq, d0, D, inf, L);
+    T ring[K][NPL];
 #pragma unroll
-    for (int j = 0; j < NPL; j++) {
-        const int d = d0 + j;
-        c[j] = d < D ? k.C[p * D + d] : inf;
-        L[j] = c[j];
-        if (d < D) Lout[p * D + d] = L[j];
-        if (REC == 2 && d < D) ck[d] = L[j];
+    for (int i = 0; i < K; i++)
+        if (1 + i < len) load_run<T, NPL, VEC>(Cq + (1 + i) * vstep, d0, D, inf, ring[i]);
+    const T* Cn = Cq + (1 + K) * vstep;  // the next load to issue
+    store_run<T, NPL, VEC>(Lq, d0, D, L);
+    if (REC == 2) store_run<T, NPL, VEC>(ck, d0, D, L);
+    T m = run_min<T, NPL>(L);
+    if (REC == 1) {
+        const int ks = run_argmin<T, NPL>(L, m, d0);
+        if (lane == 0) *kst = (uint16_t)ks;
     }
-    T m;
-    int ks;
-    warp_argmin<T, NPL>(L, d0, m, ks);
-    if (REC == 1 && lane == 0) kst[p] = (uint16_t)ks;
-    for (int t = 1; t < len; t++) {
-        x += dx;
-        y += dy;
-        p = (size_t)y * k.W + x;
+    int to_ck = k.ck;  // steps to the next checkpoint
+    for (int t0 = 1; t0 < len; t0 += K) {
 #pragma unroll
-        for (int j = 0; j < NPL; j++) {
-            const int d = d0 + j;
-            c[j] = d < D ? k.C[p * D + d] : inf;
-        }
-        uint32_t cw;
-        soft_step<T, NPL>(L, m, c, k.p1, k.p2, lane, d0, D, Ln, cw);
+        for (int i = 0; i < K; i++) {
+            if (t0 + i >= len) break;
+            T Ln[NPL];
+            uint32_t cw;
+            soft_step<T, NPL>(L, m, ring[i], k.p1, k.p2, lane, d0, D, Ln, cw);
+            if (t0 + i + K < len) load_run<T, NPL, VEC>(Cn, d0, D, inf, ring[i]);
+            Cn += vstep;
+            Lq += vstep;
 #pragma unroll
-        for (int j = 0; j < NPL; j++) {
-            const int d = d0 + j;
-            L[j] = Ln[j];
-            if (d < D) Lout[p * D + d] = L[j];
+            for (int j = 0; j < NPL; j++) L[j] = Ln[j];
+            store_run<T, NPL, VEC>(Lq, d0, D, L);
+            m = run_min<T, NPL>(L);
+            if (REC == 1) {
+                codes += pstep * 32 * CB;
+                kst += pstep;
+                store_codes<T, NPL>(codes, cw);
+                const int ks = run_argmin<T, NPL>(L, m, d0);
+                if (lane == 0) *kst = (uint16_t)ks;
+            }
+            if (REC == 2 && --to_ck == 0) {
+                to_ck = k.ck;
+                ck += D;
+                store_run<T, NPL, VEC>(ck, d0, D, L);
+            }
         }
-        if (REC == 1) store_codes<T, NPL>(codes + (p * 32 + lane) * CB, cw);
-        if (REC == 2 && t % k.ck == 0) {
-            T* dst = ck + (size_t)(t / k.ck) * D;
-#pragma unroll
-            for (int j = 0; j < NPL; j++)
-                if (d0 + j < D) dst[d0 + j] = L[j];
-        }
-        warp_argmin<T, NPL>(L, d0, m, ks);
-        if (REC == 1 && lane == 0) kst[p] = (uint16_t)ks;
     }
 }
 
 // S = sum of the directions' L in direction order, then the soft-argmin per
 // pixel (warp per pixel): stats = (Smin, 1/Z, dhat); S stored when S_out.
-template <typename T>
-__global__ void soft_argmin_kernel(const T* part, int nd, int npix, int D, T tau, T* dhat, T* stats,
-                                   T* S_out) {
+// ND directions and N = ceil(D / 32) disparities per lane are compile-time, so
+// that all ND * N loads of a pixel are in flight before the first add; with a
+// run-time direction count each load waited for the add before it (960x540,
+// D = 128, 8 directions, 2.4 GB: 1.80 ms then, 0.37 ms now, copy bandwidth).
+template <typename T, int ND, int N>
+__global__ void __launch_bounds__(256) soft_argmin_kernel(const T* part, int npix, int D, T tau, T* dhat, T* stats,
+                                                          T* S_out) {
     const int lane = threadIdx.x & 31;
     const size_t vol = (size_t)npix * D;
-    constexpr int KMAXD = 8;  // D <= 256: at most 8 disparities per lane
     for (size_t p = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < (size_t)npix;
          p += ((size_t)gridDim.x * blockDim.x) >> 5) {
-        T sv[KMAXD];
+        T v[N][ND], sv[N];
         T mn = inf_v<T>();
 #pragma unroll
-        for (int i = 0; i < KMAXD; i++) {
+        for (int i = 0; i < N; i++) {
             const int d = lane + 32 * i;
             if (d < D) {
-                T acc = part[p * D + d];
-                for (int r = 1; r < nd; r++) acc = acc + part[r * vol + p * D + d];
+                const T* q = part + p * D + d;
+#pragma unroll
+                for (int r = 0; r < ND; r++) v[i][r] = q[r * vol];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int d = lane + 32 * i;
+            if (d < D) {
+                T acc = v[i][0];
+#pragma unroll
+                for (int r = 1; r < ND; r++) acc = acc + v[i][r];
                 sv[i] = acc;
                 if (S_out) S_out[p * D + d] = acc;
                 mn = fmin(mn, acc);
@@ -279,7 +381,7 @@ __global__ void soft_argmin_kernel(const T* part, int nd, int npix, int D, T tau
         mn = warp_minv(mn);
         T z = 0, num = 0;
 #pragma unroll
-        for (int i = 0; i < KMAXD; i++) {
+        for (int i = 0; i < N; i++) {
             const int d = lane + 32 * i;
             if (d < D) {
                 const T e = exp(-(sv[i] - mn) / tau);
@@ -301,28 +403,47 @@ __global__ void soft_argmin_kernel(const T* part, int nd, int npix, int D, T tau
     }
 }
 
-// dS = g * (-1/tau) * p_d * (d - dhat)
-template <typename T>
-__global__ void soft_ds_kernel(const T* S, const T* stats, const T* g, int npix, int D, T tau, T* dS) {
-    const size_t n = (size_t)npix * D;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t p = i / D;
-        const int d = (int)(i % D);
+// dS = g * (-1/tau) * p_d * (d - dhat), a warp per pixel (no division of a
+// 64-bit cell index by D; the pixel's statistics are one broadcast load):
+// 0.26 -> 0.12 ms at 960x540, D = 128.
+template <typename T, int N>
+__global__ void __launch_bounds__(256) soft_ds_kernel(const T* S, const T* stats, const T* g, int npix, int D, T tau,
+                                                      T* dS) {
+    const int lane = threadIdx.x & 31;
+    const T c = -(T)1 / tau;
+    for (size_t p = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < (size_t)npix;
+         p += ((size_t)gridDim.x * blockDim.x) >> 5) {
+        T sv[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int d = lane + 32 * i;
+            if (d < D) sv[i] = S[p * D + d];
+        }
         const T mn = stats[3 * p], zi = stats[3 * p + 1], dh = stats[3 * p + 2];
-        const T pd = exp(-(S[i] - mn) / tau) * zi;
-        dS[i] = g[p] * (-(T)1 / tau) * pd * ((T)d - dh);
+        const T gc = g[p] * c;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const int d = lane + 32 * i;
+            if (d < D) {
+                const T pd = exp(-(sv[i] - mn) / tau) * zi;
+                dS[p * D + d] = gc * pd * ((T)d - dh);
+            }
+        }
     }
 }
 
 // Backward through one direction.  Codes and k* of the steps come from the
 // tape (CK = false) or are recomputed per k-step segment from the stored
-// checkpoints into shared memory (CK = true, k <= 32).
-template <typename T, int NPL, bool CK>
+// checkpoints into shared memory (CK = true, k <= 32).  The loads of dS (and
+// of C in the recomputation) run ahead of the walk in a register ring, as in
+// the forward pass: 2.18 -> 1.67 ms at 960x540, D = 128, checkpoints of 32,
+// where it moves 5.6 GB of DRAM (0.86 ms) and is bound by its instructions.
+template <typename T, int NPL, bool CK, bool VEC>
 __global__ void __launch_bounds__(128) soft_bwd_pass(SoftK<T> k, int nd) {
     constexpr int WARPS = 4;
     constexpr int KMAX = 32;
-    __shared__ uint16_t sk[WARPS][KMAX + 1];
-    __shared__ uint32_t segc[WARPS][KMAX][32];  // CK: codes of the segment's steps, per lane
+    __shared__ uint16_t sk[CK ? WARPS : 1][KMAX + 1];
+    __shared__ uint32_t segc[CK ? WARPS : 1][CK ? KMAX : 1][32];  // codes of the segment's steps, per lane
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int dir, wblk;
     if (!block_dir(nd, k.W, k.H, dir, wblk)) return;
@@ -337,107 +458,126 @@ __global__ void __launch_bounds__(128) soft_bwd_pass(SoftK<T> k, int nd) {
     const T inf = inf_v<T>();
     const size_t npix = (size_t)k.W * k.H;
     constexpr int CB = CodeWord<NPL>::kBytes;
-    T* dCout = k.part + (size_t)dir * npix * D;
-    const uint8_t* codes = CK ? nullptr : k.codes + (size_t)dir * npix * 32 * CB;
-    const uint16_t* kst = CK ? nullptr : k.kstar + (size_t)dir * npix;
-    const T* ckp = CK ? k.ckpt + (size_t)k.ckpt_off[(size_t)dir * (k.W + k.H) + w] * D : nullptr;
+    constexpr int K = run_ahead<T, NPL>();
+    const long long pstep = (long long)dy * k.W + dx;
+    const long long p0 = (long long)sy * k.W + sx;
+    const long long vstep = pstep * D;
+    const uint8_t* codes = CK ? nullptr : k.codes + ((size_t)dir * npix + p0) * 32 * CB + lane * CB;
+    const uint16_t* kst = CK ? nullptr : k.kstar + (size_t)dir * npix + p0;
+    const T* ckp = CK ? k.ckpt + (size_t)k.ckpt_off[(size_t)dir * (k.W + k.H) + w] * D + d0 : nullptr;
+    const T* C0 = k.C + p0 * D + d0;
+    const T* S0 = k.dS + p0 * D + d0;
+    T* O0 = k.part + ((size_t)dir * npix + p0) * D + d0;
 
     T carry[NPL];
 #pragma unroll
     for (int j = 0; j < NPL; j++) carry[j] = 0;
     T gp1 = 0, gp2 = 0;
 
-    int seg_lo = 0;  // CK: steps (seg_lo, seg_hi] have codes in segc / sk
-    int t = len - 1;
-    while (true) {
-        const int x = sx + t * dx, y = sy + t * dy;
-        const size_t p = (size_t)y * k.W + x;
-        T G[NPL];
+    // steps seg_lo+1 .. seg_hi have their codes at hand: one segment after
+    // another from the walk's end (CK), or the whole walk
+    const int seg = CK ? k.ck : len;
+    for (int seg_lo = len > 1 ? ((len - 2) / seg) * seg : 0; seg_lo >= 0; seg_lo -= seg) {
+        const int seg_hi = min(seg_lo + seg, len - 1);
+        // dS of steps seg_hi .. seg_hi-K+1; step 0 follows the first segment's last
+        const int t_end = seg_lo == 0 ? 0 : seg_lo + 1;
+        T ring[K][NPL];
 #pragma unroll
-        for (int j = 0; j < NPL; j++) {
-            const int d = d0 + j;
-            G[j] = d < D ? k.dS[p * D + d] + carry[j] : (T)0;
-            if (d < D) dCout[p * D + d] = G[j];
-        }
-        if (t == 0) break;
-        uint32_t cw;
-        int ks;
-        if (CK) {
-            if (t <= seg_lo || t == len - 1) {
-                // recompute the segment containing step t: from the checkpoint
-                // at s*k, steps s*k+1 .. min(s*k+k, len-1)
-                const int s0 = ((t - 1) / k.ck) * k.ck;
-                const int s1 = min(s0 + k.ck, len - 1);
-                T L[NPL], c[NPL], Ln[NPL];
-                const T* cl = ckp + (size_t)(s0 / k.ck) * D;
+        for (int i = 0; i < K; i++)
+            if (seg_hi - i >= t_end) load_run<T, NPL, VEC>(S0 + (seg_hi - i) * vstep, d0, D, (T)0, ring[i]);
+        if (CK && seg_hi > 0) {
+            // recompute the segment from the checkpoint at its start
+            T L[NPL], cr[K][NPL];
+            load_run<T, NPL, VEC>(ckp + (size_t)(seg_lo / seg) * D, d0, D, inf, L);
+            const T* Cu = C0 + (seg_lo + 1) * vstep;
 #pragma unroll
-                for (int j = 0; j < NPL; j++) L[j] = (d0 + j < D) ? cl[d0 + j] : inf;
-                T m;
-                int kk;
-                warp_argmin<T, NPL>(L, d0, m, kk);
-                if (lane == 0) sk[warp][0] = (uint16_t)kk;
-#pragma unroll 1
-                for (int u = s0 + 1; u <= s1; u++) {
-                    const int xu = sx + u * dx, yu = sy + u * dy;
-                    const size_t pu = (size_t)yu * k.W + xu;
+            for (int i = 0; i < K; i++)
+                if (seg_lo + 1 + i <= seg_hi) load_run<T, NPL, VEC>(Cu + i * vstep, d0, D, inf, cr[i]);
+            const T* Cn = Cu + K * vstep;
+            T m = run_min<T, NPL>(L);
+            int kk = run_argmin<T, NPL>(L, m, d0);
+            __syncwarp();  // the previous segment's codes have been read
+            if (lane == 0) sk[warp][0] = (uint16_t)kk;
+            for (int u0 = seg_lo + 1; u0 <= seg_hi; u0 += K) {
 #pragma unroll
-                    for (int j = 0; j < NPL; j++) c[j] = (d0 + j < D) ? k.C[pu * D + d0 + j] : inf;
+                for (int i = 0; i < K; i++) {
+                    const int u = u0 + i;
+                    if (u > seg_hi) break;
+                    T Ln[NPL];
                     uint32_t cwu;
-                    soft_step<T, NPL>(L, m, c, k.p1, k.p2, lane, d0, D, Ln, cwu);
+                    soft_step<T, NPL>(L, m, cr[i], k.p1, k.p2, lane, d0, D, Ln, cwu);
+                    if (u + K <= seg_hi) load_run<T, NPL, VEC>(Cn, d0, D, inf, cr[i]);
+                    Cn += vstep;
+                    segc[warp][u - seg_lo - 1][lane] = cwu;
+                    if (u == seg_hi) break;  // the last step's L and argmin are not needed
 #pragma unroll
                     for (int j = 0; j < NPL; j++) L[j] = Ln[j];
-                    segc[warp][u - s0 - 1][lane] = cwu;
-                    warp_argmin<T, NPL>(L, d0, m, kk);
-                    if (lane == 0 && u - s0 < KMAX + 1) sk[warp][u - s0] = (uint16_t)kk;
+                    m = run_min<T, NPL>(L);
+                    kk = run_argmin<T, NPL>(L, m, d0);
+                    if (lane == 0) sk[warp][u - seg_lo] = (uint16_t)kk;
                 }
-                __syncwarp();
-                seg_lo = s0;
             }
-            cw = segc[warp][t - seg_lo - 1][lane];
-            ks = sk[warp][t - 1 - seg_lo];
-        } else {
-            cw = load_codes<T, NPL>(codes + (p * 32 + lane) * CB);
-            const int xp = x - dx, yp = y - dy;
-            ks = kst[(size_t)yp * k.W + xp];
+            __syncwarp();
         }
-        // neighbours' G and codes
-        T gup = __shfl_up_sync(FULLM, G[NPL - 1], 1);
-        T gdn = __shfl_down_sync(FULLM, G[0], 1);
-        uint32_t cup = __shfl_up_sync(FULLM, cw >> (2 * (NPL - 1)), 1) & 3u;
-        uint32_t cdn = __shfl_down_sync(FULLM, cw, 1) & 3u;
-        if (lane == 0) {
-            gup = 0;
-            cup = 0;
-        }
-        if (lane == 31) {
-            gdn = 0;
-            cdn = 0;
-        }
-        T gs = 0, g3 = 0;
+        for (int t0 = seg_hi; t0 >= t_end; t0 -= K) {
 #pragma unroll
-        for (int j = 0; j < NPL; j++) {
-            const uint32_t cj = (cw >> (2 * j)) & 3u;
-            gs += G[j];
-            if (cj == 3u) g3 += G[j];
-            if (cj == 1u || cj == 2u) gp1 += G[j];
-        }
-        gp2 += g3;
-        const T gm = warp_sum(g3 - gs);
+            for (int i = 0; i < K; i++) {
+                const int t = t0 - i;
+                if (t < t_end) break;
+                T G[NPL];
 #pragma unroll
-        for (int j = 0; j < NPL; j++) {
-            const uint32_t cj = (cw >> (2 * j)) & 3u;
-            const uint32_t cplus = j < NPL - 1 ? (cw >> (2 * (j + 1))) & 3u : cdn;
-            const uint32_t cminus = j > 0 ? (cw >> (2 * (j - 1))) & 3u : cup;
-            const T gplus = j < NPL - 1 ? G[j + 1] : gdn;
-            const T gminus = j > 0 ? G[j - 1] : gup;
-            T v = 0;
-            if (cj == 0u) v += G[j];
-            if (cplus == 1u) v += gplus;
-            if (cminus == 2u) v += gminus;
-            if (d0 + j == ks) v += gm;
-            carry[j] = v;
+                for (int j = 0; j < NPL; j++) G[j] = d0 + j < D ? ring[i][j] + carry[j] : (T)0;
+                if (t - K >= t_end) load_run<T, NPL, VEC>(S0 + (t - K) * vstep, d0, D, (T)0, ring[i]);
+                store_run<T, NPL, VEC>(O0 + t * vstep, d0, D, G);
+                if (t == 0) break;
+                uint32_t cw;
+                int ks;
+                if (CK) {
+                    cw = segc[warp][t - seg_lo - 1][lane];
+                    ks = sk[warp][t - 1 - seg_lo];
+                } else {
+                    cw = load_codes<T, NPL>(codes + t * pstep * 32 * CB);
+                    ks = kst[(t - 1) * pstep];
+                }
+                // neighbours' G and codes
+                T gup = __shfl_up_sync(FULLM, G[NPL - 1], 1);
+                T gdn = __shfl_down_sync(FULLM, G[0], 1);
+                uint32_t cup = __shfl_up_sync(FULLM, cw >> (2 * (NPL - 1)), 1) & 3u;
+                uint32_t cdn = __shfl_down_sync(FULLM, cw, 1) & 3u;
+                if (lane == 0) {
+                    gup = 0;
+                    cup = 0;
+                }
+                if (lane == 31) {
+                    gdn = 0;
+                    cdn = 0;
+                }
+                T gs = 0, g3 = 0;
+#pragma unroll
+                for (int j = 0; j < NPL; j++) {
+                    const uint32_t cj = (cw >> (2 * j)) & 3u;
+                    gs += G[j];
+                    if (cj == 3u) g3 += G[j];
+                    if (cj == 1u || cj == 2u) gp1 += G[j];
+                }
+                gp2 += g3;
+                const T gm = warp_sum(g3 - gs);
+#pragma unroll
+                for (int j = 0; j < NPL; j++) {
+                    const uint32_t cj = (cw >> (2 * j)) & 3u;
+                    const uint32_t cplus = j < NPL - 1 ? (cw >> (2 * (j + 1))) & 3u : cdn;
+                    const uint32_t cminus = j > 0 ? (cw >> (2 * (j - 1))) & 3u : cup;
+                    const T gplus = j < NPL - 1 ? G[j + 1] : gdn;
+                    const T gminus = j > 0 ? G[j - 1] : gup;
+                    T v = 0;
+                    if (cj == 0u) v += G[j];
+                    if (cplus == 1u) v += gplus;
+                    if (cminus == 2u) v += gminus;
+                    if (d0 + j == ks) v += gm;
+                    carry[j] = v;
+                }
+            }
         }
-        t--;
     }
     gp1 = warp_sum(gp1);
     gp2 = warp_sum(gp2);
@@ -448,29 +588,57 @@ __global__ void __launch_bounds__(128) soft_bwd_pass(SoftK<T> k, int nd) {
     }
 }
 
-// dP = sum of the per-walk partials in a fixed order (deterministic).
+// dP = sum of the per-walk partials in a fixed order (deterministic): lane l
+// adds the walks l, l + 32, ... of one direction after another; the loads of
+// eight walks are in flight ahead of the adds.
 template <typename T>
-__global__ void soft_pen_reduce(const T* part, int ndir, int W, int H, T* dpen) {
+__device__ void soft_pen_reduce(const T* part, int ndir, int W, int H, T* dpen) {
     const int lane = threadIdx.x & 31;
     const int which = threadIdx.x >> 5;  // 0: P1, 1: P2
     if (which > 1) return;
     T acc = 0;
     for (int d = 0; d < ndir; d++) {
-        const int dx = d == 2 || d == 3 ? 0 : 1, dy = d < 2 ? 0 : 1;
-        const int nw = dy == 0 ? H : (dx == 0 ? W : W + H - 1);
-        for (int w = lane; w < nw; w += 32) acc += part[((size_t)d * (W + H) + w) * 2 + which];
+        const int nw = nwalks_dev(kSoftDx[d], kSoftDy[d], W, H);
+        const T* q = part + (size_t)d * (W + H) * 2 + which;
+        for (int w0 = lane; w0 < nw; w0 += 256) {
+            T v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (w0 + 32 * i < nw) v[i] = q[(size_t)(w0 + 32 * i) * 2];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (w0 + 32 * i < nw) acc += v[i];
+        }
     }
     acc = warp_sum(acc);
     if (lane == 0) dpen[which] = acc;
 }
 
-// dC = sum of the directions' contributions in direction order.
-template <typename T>
-__global__ void soft_dc_sum(const T* part, int nd, size_t vol, T* dC) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += (size_t)gridDim.x * blockDim.x) {
-        T acc = part[i];
-        for (int r = 1; r < nd; r++) acc = acc + part[r * vol + i];
-        dC[i] = acc;
+// dC = sum of the directions' contributions in direction order (E elements
+// per thread in one vector, all directions' loads in flight: 0.49 -> 0.35 ms
+// at 960x540, D = 128, copy bandwidth); the last block reduces the penalties'
+// per-walk sums, which were a launch of one block behind this one (0.03 ms).
+template <typename T, int ND, int E>
+__global__ void __launch_bounds__(256) soft_dc_sum(const T* part, size_t vol, T* dC, const T* pen_part, int W, int H,
+                                                   T* dpen) {
+    struct alignas(E * sizeof(T)) Chunk {
+        T e[E];
+    };
+    if (blockIdx.x == gridDim.x - 1) {
+        soft_pen_reduce<T>(pen_part, ND, W, H, dpen);
+        return;
+    }
+    const size_t n = vol / E, stride = (size_t)(gridDim.x - 1) * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        Chunk v[ND];
+#pragma unroll
+        for (int r = 0; r < ND; r++) v[r] = reinterpret_cast<const Chunk*>(part + r * vol)[i];
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+#pragma unroll
+            for (int r = 1; r < ND; r++) v[0].e[j] = v[0].e[j] + v[r].e[j];
+        }
+        reinterpret_cast<Chunk*>(dC)[i] = v[0];
     }
 }
 
@@ -488,29 +656,39 @@ int soft_blocks(int nd, int W, int H) {
     return b;
 }
 
-template <typename T, int NPL>
+template <typename T, int NPL, bool VEC>
 cudaError_t fwd_all(SoftK<T> k, int paths, int rec, cudaStream_t st, Timer* tm) {
     const int nd = paths == 4 ? 4 : 8;
     const int blocks = soft_blocks(nd, k.W, k.H);
-    if (rec == 0) soft_fwd_pass<T, NPL, 0><<<blocks, 128, 0, st>>>(k, nd);
-    else if (rec == 1) soft_fwd_pass<T, NPL, 1><<<blocks, 128, 0, st>>>(k, nd);
-    else soft_fwd_pass<T, NPL, 2><<<blocks, 128, 0, st>>>(k, nd);
+    if (rec == 0) soft_fwd_pass<T, NPL, 0, VEC><<<blocks, 128, 0, st>>>(k, nd);
+    else if (rec == 1) soft_fwd_pass<T, NPL, 1, VEC><<<blocks, 128, 0, st>>>(k, nd);
+    else soft_fwd_pass<T, NPL, 2, VEC><<<blocks, 128, 0, st>>>(k, nd);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (tm) tm->mark("soft_fwd_pass");
     return cudaSuccess;
 }
 
-template <typename T, int NPL>
+template <typename T, int NPL, bool VEC>
 cudaError_t bwd_all(SoftK<T> k, int paths, bool ck, cudaStream_t st, Timer* tm) {
     const int nd = paths == 4 ? 4 : 8;
     const int blocks = soft_blocks(nd, k.W, k.H);
-    if (ck) soft_bwd_pass<T, NPL, true><<<blocks, 128, 0, st>>>(k, nd);
-    else soft_bwd_pass<T, NPL, false><<<blocks, 128, 0, st>>>(k, nd);
+    if (ck) soft_bwd_pass<T, NPL, true, VEC><<<blocks, 128, 0, st>>>(k, nd);
+    else soft_bwd_pass<T, NPL, false, VEC><<<blocks, 128, 0, st>>>(k, nd);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (tm) tm->mark("soft_bwd_pass");
     return cudaSuccess;
+}
+
+// Whole-vector accesses: every pixel's run of D values starts on 16 bytes and
+// a lane's values never straddle its end.
+template <typename T>
+bool runs_aligned(int D, int npl, std::initializer_list<const void*> ptrs) {
+    if (D % npl != 0 || (D * sizeof(T)) % 16 != 0) return false;
+    for (const void* p : ptrs)
+        if ((uintptr_t)p & 15) return false;
+    return true;
 }
 
 int grid_for(size_t n, int block) {
@@ -536,14 +714,34 @@ cudaError_t soft_forward_t(const SoftLaunch& L, cudaStream_t st, Timer* tm) {
     k.p2 = (T)L.p2;
     const int rec = L.record ? (L.ck > 0 ? 2 : 1) : 0;
     cudaError_t e;
-    if (L.D <= 32) e = fwd_all<T, 1>(k, L.paths, rec, st, tm);
-    else if (L.D <= 64) e = fwd_all<T, 2>(k, L.paths, rec, st, tm);
-    else if (L.D <= 128) e = fwd_all<T, 4>(k, L.paths, rec, st, tm);
-    else e = fwd_all<T, 8>(k, L.paths, rec, st, tm);
+    const int npl = L.D <= 32 ? 1 : (L.D <= 64 ? 2 : (L.D <= 128 ? 4 : 8));
+    if (runs_aligned<T>(L.D, npl, {L.cost, L.part, L.ckpt})) {
+        if (npl == 1) e = fwd_all<T, 1, true>(k, L.paths, rec, st, tm);
+        else if (npl == 2) e = fwd_all<T, 2, true>(k, L.paths, rec, st, tm);
+        else if (npl == 4) e = fwd_all<T, 4, true>(k, L.paths, rec, st, tm);
+        else e = fwd_all<T, 8, true>(k, L.paths, rec, st, tm);
+    } else {
+        if (npl == 1) e = fwd_all<T, 1, false>(k, L.paths, rec, st, tm);
+        else if (npl == 2) e = fwd_all<T, 2, false>(k, L.paths, rec, st, tm);
+        else if (npl == 4) e = fwd_all<T, 4, false>(k, L.paths, rec, st, tm);
+        else e = fwd_all<T, 8, false>(k, L.paths, rec, st, tm);
+    }
     if (e != cudaSuccess) return e;
     const int npix = L.W * L.H;
-    soft_argmin_kernel<T><<<grid_for((size_t)npix * 32, 256), 256, 0, st>>>(
-        (const T*)L.part, L.paths == 4 ? 4 : 8, npix, L.D, (T)L.tau, (T*)L.dhat, (T*)L.stats, (T*)L.S);
+    const int grid = grid_for((size_t)npix * 32, 256);
+    auto argmin = [&](auto nc) {
+        constexpr int N = decltype(nc)::value;
+        if (L.paths == 4)
+            soft_argmin_kernel<T, 4, N><<<grid, 256, 0, st>>>((const T*)L.part, npix, L.D, (T)L.tau, (T*)L.dhat,
+                                                              (T*)L.stats, (T*)L.S);
+        else
+            soft_argmin_kernel<T, 8, N><<<grid, 256, 0, st>>>((const T*)L.part, npix, L.D, (T)L.tau, (T*)L.dhat,
+                                                              (T*)L.stats, (T*)L.S);
+    };
+    if (npl == 1) argmin(std::integral_constant<int, 1>{});
+    else if (npl == 2) argmin(std::integral_constant<int, 2>{});
+    else if (npl == 4) argmin(std::integral_constant<int, 4>{});
+    else argmin(std::integral_constant<int, 8>{});
     if (tm) tm->mark("soft_argmin");
     return cudaGetLastError();
 }
@@ -568,22 +766,46 @@ cudaError_t soft_backward_t(const SoftLaunch& L, cudaStream_t st, Timer* tm) {
     k.dpen_part = (T*)L.dpen_part;
     const int npix = L.W * L.H;
     cudaError_t e;
-    soft_ds_kernel<T><<<grid_for((size_t)npix * L.D, 256), 256, 0, st>>>(
-        (const T*)L.S, (const T*)L.stats, (const T*)L.g, npix, L.D, (T)L.tau, (T*)L.dS);
+    const int npl = L.D <= 32 ? 1 : (L.D <= 64 ? 2 : (L.D <= 128 ? 4 : 8));
+    const int wgrid = grid_for((size_t)npix * 32, 256);
+    auto ds = [&](auto nc) {
+        soft_ds_kernel<T, decltype(nc)::value><<<wgrid, 256, 0, st>>>((const T*)L.S, (const T*)L.stats, (const T*)L.g,
+                                                                      npix, L.D, (T)L.tau, (T*)L.dS);
+    };
+    if (npl == 1) ds(std::integral_constant<int, 1>{});
+    else if (npl == 2) ds(std::integral_constant<int, 2>{});
+    else if (npl == 4) ds(std::integral_constant<int, 4>{});
+    else ds(std::integral_constant<int, 8>{});
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (tm) tm->mark("soft_dS");
     const bool ck = L.ck > 0;
-    if (L.D <= 32) e = bwd_all<T, 1>(k, L.paths, ck, st, tm);
-    else if (L.D <= 64) e = bwd_all<T, 2>(k, L.paths, ck, st, tm);
-    else if (L.D <= 128) e = bwd_all<T, 4>(k, L.paths, ck, st, tm);
-    else e = bwd_all<T, 8>(k, L.paths, ck, st, tm);
+    if (runs_aligned<T>(L.D, npl, {L.cost, L.part, L.dS, L.ckpt})) {
+        if (npl == 1) e = bwd_all<T, 1, true>(k, L.paths, ck, st, tm);
+        else if (npl == 2) e = bwd_all<T, 2, true>(k, L.paths, ck, st, tm);
+        else if (npl == 4) e = bwd_all<T, 4, true>(k, L.paths, ck, st, tm);
+        else e = bwd_all<T, 8, true>(k, L.paths, ck, st, tm);
+    } else {
+        if (npl == 1) e = bwd_all<T, 1, false>(k, L.paths, ck, st, tm);
+        else if (npl == 2) e = bwd_all<T, 2, false>(k, L.paths, ck, st, tm);
+        else if (npl == 4) e = bwd_all<T, 4, false>(k, L.paths, ck, st, tm);
+        else e = bwd_all<T, 8, false>(k, L.paths, ck, st, tm);
+    }
     if (e != cudaSuccess) return e;
     const size_t vol = (size_t)npix * L.D;
-    soft_dc_sum<T><<<grid_for(vol, 256), 256, 0, st>>>((const T*)L.part, L.paths == 4 ? 4 : 8, vol, (T*)L.dcost);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    constexpr int E = 16 / (int)sizeof(T);
+    auto dc = [&](auto ndc, auto ec) {
+        constexpr int ND = decltype(ndc)::value, EE = decltype(ec)::value;
+        soft_dc_sum<T, ND, EE><<<grid_for(vol / EE + 1, 256) + 1, 256, 0, st>>>(
+            (const T*)L.part, vol, (T*)L.dcost, k.dpen_part, L.W, L.H, k.dpen);
+    };
+    using i4 = std::integral_constant<int, 4>;
+    using i8 = std::integral_constant<int, 8>;
+    using one = std::integral_constant<int, 1>;
+    using vec = std::integral_constant<int, E>;
+    const bool dvec = vol % E == 0 && (((uintptr_t)L.part | (uintptr_t)L.dcost) & 15) == 0;
+    if (L.paths == 4) dvec ? dc(i4{}, vec{}) : dc(i4{}, one{});
+    else dvec ? dc(i8{}, vec{}) : dc(i8{}, one{});
     if (tm) tm->mark("soft_dc_sum");
-    soft_pen_reduce<T><<<1, 64, 0, st>>>(k.dpen_part, L.paths == 4 ? 4 : 8, L.W, L.H, k.dpen);
-    if (tm) tm->mark("soft_pen_reduce");
     return cudaGetLastError();
 }
 

@@ -95,8 +95,8 @@ def config(sem):
             "max_disp": D, "paths": PATHS, "p1": P1, "p2": P2, "p2_mode": "constant",
             "recurrence": s["recurrence"], "path_table": s["table"],
             "domain": "u8 intensities used unscaled", "lr_threshold": LR,
-            "l2": "a timed frame sequence has no flush between frames: every frame streams 15.5 GB of "
-                  "aggregation volumes through HBM (126 MB L2) and an input pair recurs only after three "
+            "l2": "a timed frame sequence has no flush between frames: every frame streams 8.5 GB of "
+                  "per-direction volumes through HBM (126 MB L2) and an input pair recurs only after three "
                   "other frames; one-frame-per-call legs flush L2 (256 MiB write) before each call",
             "inputs": "seeded synthetic video frames (moving rectangles over a slanted plane)"}
 
@@ -861,26 +861,19 @@ def measure_video(ctx, dev, n_frames=300, refit_steps=50):
 
 # ------------------------------------------------------------------ ours
 def kernel_of(sem):
-    """The compiled kernel behind each timed pass (PPL = 4 at D = 256), as
-    ncu names it; the last template argument is the kernel variant."""
-    e = SEMANTICS[sem]["var"]
+    """The compiled kernel behind each timed launch (32 lanes per line at
+    D = 256), as ncu names it."""
+    excl = 1 if SEMANTICS[sem]["var"] >= 2 else 0  # the CPU recurrence's minimum without d = D-1
     return {
-        "fused_prep": "prep_kernel",
-        "fused_pass_V+": f"vd_pass<4, 0, 0, {e}>",
-        "fused_pass_D1-": f"vd_pass<4, 0, 1, {e}>",
-        "fused_pass_V-": f"vd_pass<4, 1, 0, {e}>",
-        "fused_pass_D1+": f"vd_pass<4, 1, 1, {e}>",
-        "fused_pass_D2+": f"vd_pass<4, 1, 1, {e}>",
-        "fused_pass_D2-": f"vd_pass<4, 1, 1, {e}>",
-        "fused_pass_H+": f"hp_pass<4, 1, 1, {e}>",
-        "fused_pass_H-_wta": f"hp_wta_pass<4, 0, {e}>",
+        "fused_prep": "dirs_prep_kernel",
+        "fused_pass_H-H+V-V+D": f"dirs_pass_kernel<32, 2, {excl}>",
+        "fused_sum_wta": f"dirs_sum_kernel<32, 8, {0 if SEMANTICS[sem]['var'] == 0 else 1}, {excl}, 1>",
     }
 
 
 def time_frames(ctx, frames, kw, steps, flush, st):
     """Device ms per frame of tdv_stereo_sgm over device-resident frames, L2
-    flushed before each, and the per-kernel means (events around each kernel,
-    the two pass chains in sequence)."""
+    flushed before each, and the per-kernel means (events around each kernel)."""
     import ctypes
 
     import torch
@@ -953,24 +946,18 @@ def measure_reference_literal(ctx, dev, frames, flush, reps=5):
 
 def alg_bytes(name):
     """Algorithmic HBM bytes of one launch of a fused kernel at this size:
-    the u16 aggregation volumes (256 disparities = 512 B per pixel) read
-    and/or written once, plus the 16-byte BT planes of both images once.  At
-    8 paths the passes run as two concurrent chains on two volumes (V+ V- D1+
-    and D1- D2+ D2-): V+ and D1- only store their volume, the other chain
-    passes read and write it, H+ reads both and writes the first, H- reads it
-    and writes the maps."""
+    one byte per cell (256 per pixel) and direction, written by the pass and
+    read by the sum, plus the 16-byte BT planes of both images once; the
+    CPU recurrence's last two disparities (4 bytes per pixel and direction)
+    are not counted."""
     pix = W * H
-    s_vol = pix * 256 * 2
+    vols = PATHS * pix * 256
     planes = 2 * pix * 16
     if name == "fused_prep":
         return 2 * pix + planes
-    if name in ("fused_pass_V+", "fused_pass_D1-"):
-        return s_vol + planes
-    if name == "fused_pass_H+":
-        return 3 * s_vol + planes
-    if name.endswith("_wta"):
-        return s_vol + planes + 3 * pix * 2
-    return 2 * s_vol + planes
+    if name == "fused_sum_wta":
+        return vols + planes + 3 * pix * 2
+    return vols + planes
 
 
 def run_ours(args):
@@ -1185,7 +1172,7 @@ def run_ours(args):
         "single_frame": {"value": frames / (single_ms / 1000.0), "unit": UNIT,
                          "ms_per_frame": single_ms / args.steps, "clocks": clocks_single,
                          "path": "one tdv_stereo_sgm call per frame, L2 flushed before each; the per-frame "
-                                 "latency (the two pass chains of a frame run concurrently)"},
+                                 "latency"},
         "e2e": {"value": stream_fps, "unit": UNIT, "h2d_bytes_per_step": 2 * W * H,
                 "d2h_bytes_per_step": 2 * W * H, "ms_per_step": stream_ms / args.steps,
                 "path": "video.VideoLoop: pinned host frames in, maps out to pinned host, two buffer sets, "

@@ -83,10 +83,22 @@ void release_buf(tdv_ctx* ctx, tdv_ctx::Buf& b) {
 
 cudaStream_t S(tdv_stream s) { return (cudaStream_t)s; }
 
+// Scratch of the directions stored apart, where the allocator has room for it:
+// false sends the call to the accumulating passes, which need a quarter to a
+// half of it.
+bool dirs_ready(tdv_ctx* ctx, tdv_ctx::Buf& b, int W, int H, int D, int paths, int excl) {
+    const size_t n = tdv::dirs_bytes(W, H, D, paths, excl);
+    if (b.bytes >= n) return true;
+    if (n >= ctx->dirs_refused) return false;
+    if (ensure(ctx, b, n) == TDV_OK) return true;
+    ctx->dirs_refused = n;
+    return false;
+}
+
 // Scratch of the fused path for pairs up to W x H x D: planes and both
 // aggregation volumes.
 tdv_status reserve_fused(tdv_ctx* ctx, int W, int H, int D) {
-    TDV_TRY(ensure(ctx, ctx->planes, tdv::fused_plane_bytes(W, H)));
+    TDV_TRY(ensure(ctx, ctx->planes, std::max(tdv::fused_plane_bytes(W, H), tdv::dirs_plane_bytes(W, H))));
     if (D <= tdv::kMaxDispSgm) {
         TDV_TRY(ensure(ctx, ctx->agg, tdv::fused_agg_bytes(W, H, D)));
         TDV_TRY(ensure(ctx, ctx->agg2, tdv::fused_agg_bytes(W, H, D)));
@@ -474,7 +486,8 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
     const bool any = ctx->agg.ptr || ctx->cost.ptr || ctx->planes.ptr || ctx->codes.ptr ||
                      ctx->misc.ptr || ctx->sched_buf.ptr || ctx->err.ptr || ctx->soft.ptr ||
                      ctx->agg2.ptr || ctx->defer.ptr || ctx->side || ctx->fw_buf.ptr || ctx->fside.ptr ||
-                     ctx->lane_main || ctx->planes_b.ptr || ctx->agg_b.ptr || ctx->agg2_b.ptr || ctx->fside_b.ptr;
+                     ctx->lane_main || ctx->planes_b.ptr || ctx->agg_b.ptr || ctx->agg2_b.ptr || ctx->fside_b.ptr ||
+                     ctx->dirs.ptr || ctx->dirs_b.ptr;
     if (any) {
         DeviceScope ds(ctx->device);
         cudaDeviceSynchronize();
@@ -497,6 +510,8 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
         release_buf(ctx, ctx->agg_b);
         release_buf(ctx, ctx->agg2_b);
         release_buf(ctx, ctx->fside_b);
+        release_buf(ctx, ctx->dirs);
+        release_buf(ctx, ctx->dirs_b);
         if (ctx->lane_main) cudaStreamDestroy(ctx->lane_main);
         if (ctx->lane_side) cudaStreamDestroy(ctx->lane_side);
         for (cudaEvent_t e : {ctx->lane_fork, ctx->lane_join, ctx->lane_start, ctx->lane_done})
@@ -514,7 +529,7 @@ tdv_status tdv_ctx_set_allocator(tdv_ctx* ctx, tdv_alloc_fn alloc, tdv_free_fn r
     if ((alloc == nullptr) != (release == nullptr))
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator and release must be set together");
     if (ctx->agg.ptr || ctx->cost.ptr || ctx->planes.ptr || ctx->codes.ptr || ctx->misc.ptr ||
-        ctx->sched_buf.ptr || ctx->defer.ptr)
+        ctx->sched_buf.ptr || ctx->defer.ptr || ctx->dirs.ptr || ctx->dirs_b.ptr)
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator must be set before any scratch exists");
     ctx->alloc = alloc;
     ctx->release = release;
@@ -526,11 +541,16 @@ tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t W, int32_t H, int32_t D) {
     if (!ctx) return TDV_ERR_INVALID_ARG;
     if (W <= 0 || H <= 0 || D <= 0 || W > kMaxSide || H > kMaxSide)
         return fail(ctx, TDV_ERR_INVALID_ARG, "bad reserve size %dx%dx%d", W, H, D);
+    auto reserve = [&]() -> tdv_status {
+        TDV_TRY(reserve_fused(ctx, W, H, D));
+        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1);
+        return TDV_OK;
+    };
     if (!ctx->alloc) {
         TDV_DEVICE_SCOPE(ctx);
-        return reserve_fused(ctx, W, H, D);
+        return reserve();
     }
-    return reserve_fused(ctx, W, H, D);
+    return reserve();
 }
 
 tdv_status tdv_ctx_enable_timing(tdv_ctx* ctx, int32_t enable) {
@@ -864,6 +884,16 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         fused = fused_weights_ready(ctx, W, H, D, params, fp, S(stream), &werr);
         TDV_TRY(werr);
     }
+    if (fused && tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
+        dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl)) {
+        TDV_TRY(ensure(ctx, ctx->planes, tdv::dirs_plane_bytes(W, H)));
+        TDV_TRY(ensure_err(ctx, S(stream)));
+        tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
+        a.planes = ctx->planes.ptr;
+        a.agg = ctx->dirs.ptr;
+        TDV_CUDA(tdv::launch_dirs(a, S(stream), &ctx->timer));
+        return TDV_OK;
+    }
     if (fused) {
         TDV_TRY(reserve_fused(ctx, W, H, D));
         TDV_TRY(ensure_side(ctx));
@@ -925,15 +955,24 @@ tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left,
         if (!ok)
             return fail(ctx, TDV_ERR_UNSUPPORTED, "this size, table and semantics leave the fused path's ranges");
     }
-    TDV_TRY(reserve_fused(ctx, W, H, D));
-    TDV_TRY(ensure_side(ctx));
+    const bool dirs = tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
+                      dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl) &&
+                      (n == 1 || dirs_ready(ctx, ctx->dirs_b, W, H, D, params->paths, fp.excl));
+    if (dirs) {
+        TDV_TRY(ensure(ctx, ctx->planes, tdv::dirs_plane_bytes(W, H)));
+    } else {
+        TDV_TRY(reserve_fused(ctx, W, H, D));
+        TDV_TRY(ensure_side(ctx));
+    }
     TDV_TRY(ensure_err(ctx, st));
     if (n > 1) {
         TDV_TRY(ensure_lane(ctx));
-        TDV_TRY(ensure(ctx, ctx->planes_b, tdv::fused_plane_bytes(W, H)));
-        TDV_TRY(ensure(ctx, ctx->agg_b, tdv::fused_agg_bytes(W, H, D)));
-        TDV_TRY(ensure(ctx, ctx->agg2_b, tdv::fused_agg_bytes(W, H, D)));
-        if (fp.weighted && ctx->fside.bytes) TDV_TRY(ensure(ctx, ctx->fside_b, ctx->fside.bytes));
+        TDV_TRY(ensure(ctx, ctx->planes_b, dirs ? tdv::dirs_plane_bytes(W, H) : tdv::fused_plane_bytes(W, H)));
+        if (!dirs) {
+            TDV_TRY(ensure(ctx, ctx->agg_b, tdv::fused_agg_bytes(W, H, D)));
+            TDV_TRY(ensure(ctx, ctx->agg2_b, tdv::fused_agg_bytes(W, H, D)));
+            if (fp.weighted && ctx->fside.bytes) TDV_TRY(ensure(ctx, ctx->fside_b, ctx->fside.bytes));
+        }
         // the second lane starts after what the call's stream holds
         TDV_CUDA(cudaEventRecord(ctx->lane_start, st));
         TDV_CUDA(cudaStreamWaitEvent(ctx->lane_main, ctx->lane_start, 0));
@@ -942,6 +981,11 @@ tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left,
         tdv::FusedArgs a = fused_args(ctx, &left[i], &right[i], D, params, fp, &out[i]);
         const bool b = (i & 1) != 0;
         a.planes = b ? ctx->planes_b.ptr : ctx->planes.ptr;
+        if (dirs) {
+            a.agg = b ? ctx->dirs_b.ptr : ctx->dirs.ptr;
+            TDV_CUDA(tdv::launch_dirs(a, b ? ctx->lane_main : st, nullptr));
+            continue;
+        }
         a.agg = b ? ctx->agg_b.ptr : ctx->agg.ptr;
         a.agg2 = b ? ctx->agg2_b.ptr : ctx->agg2.ptr;
         if (fp.weighted) a.side = (uint32_t*)(b ? ctx->fside_b.ptr : ctx->fside.ptr);

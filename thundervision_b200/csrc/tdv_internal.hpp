@@ -186,6 +186,11 @@ struct tdv_ctx {
     // lane's planes, volumes and side rows, its two streams, its chains'
     // fork/join events and the events that tie it to the call's stream
     Buf planes_b, agg_b, agg2_b, fside_b;
+    // fused path with the directions stored apart (kernels_dirs.cu), per lane;
+    // dirs_refused: the smallest such request the allocator turned down, so
+    // that later calls of that size go straight to the accumulating passes
+    Buf dirs, dirs_b;
+    size_t dirs_refused = (size_t)-1;
     cudaStream_t lane_main = nullptr, lane_side = nullptr;
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr, lane_start = nullptr, lane_done = nullptr;
 };
@@ -304,6 +309,15 @@ cudaError_t launch_reproject(const RasterArg& disp, const RasterArg* color, int 
                              const float* q, float* verts, float* cols, cudaStream_t st);
 size_t fused_plane_bytes(int W, int H);
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t st, Timer* tm);
+
+// The same call with every direction stored apart as one byte per cell
+// (kernels_dirs.cu): FusedArgs with `planes` of dirs_plane_bytes() and `agg`
+// of dirs_bytes(); agg2, the side stream and events, off_h and side are not
+// used.
+bool dirs_supported(int W, int H, int D, int p1h, int p2h, int excl);
+size_t dirs_plane_bytes(int W, int H);
+size_t dirs_bytes(int W, int H, int D, int paths, int excl);
+cudaError_t launch_dirs(const FusedArgs& a, cudaStream_t st, Timer* tm);
 
 // Batched fused path (kernels_batch.cu): one persistent launch for many
 // integer-domain pairs of uneven size and disparity range.

@@ -165,10 +165,14 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
     if (!tdv::build_schedule(W, H, table, paths, fresh))
         return fail(ctx, TDV_ERR_BAD_WORK, "path table for %dx%d has a walk outside the image", W, H);
     const size_t wbytes = (fresh.walks.size() * sizeof(tdv::Walk) + 255) & ~(size_t)255;
-    TDV_TRY(ensure(ctx, ctx->sched_buf, wbytes + (fresh.deferred.size() + 1) * sizeof(int32_t)));
+    const size_t dbytes = ((fresh.deferred.size() + 1) * sizeof(int32_t) + 255) & ~(size_t)255;
+    TDV_TRY(ensure(ctx, ctx->sched_buf, wbytes + dbytes + fresh.mult.size() * sizeof(uint16_t)));
     sc = std::move(fresh);
     sc.d_walks = (tdv::Walk*)ctx->sched_buf.ptr;
     sc.d_deferred = (int32_t*)((char*)ctx->sched_buf.ptr + wbytes);
+    sc.d_mult = (uint16_t*)((char*)ctx->sched_buf.ptr + wbytes + dbytes);
+    TDV_CUDA(cudaMemcpyAsync(sc.d_mult, sc.mult.data(), sc.mult.size() * sizeof(uint16_t), cudaMemcpyHostToDevice,
+                             st));
     TDV_CUDA(cudaMemcpyAsync(sc.d_walks, sc.walks.data(), sc.walks.size() * sizeof(tdv::Walk),
                              cudaMemcpyHostToDevice, st));
     if (!sc.deferred.empty())
@@ -179,27 +183,32 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
     return TDV_OK;
 }
 
+// How many of the general path's passes run side by side, each with a volume
+// of its own: all of them while their volumes stay within 10 GB, else four (a
+// group then also reads and writes S once, 8 bytes per cell beside 48); 0 where
+// the allocator has no room for them (the passes then run in sequence on S).
+int side_by_side(tdv_ctx* ctx, int W, int H, int D) {
+    const size_t vol = tdv::sgm_dirs_volume(W, H, D);
+    const int np = (int)ctx->sched.passes.size();
+    const int all = std::min(np, tdv::kMaxSideBySide);
+    for (int g : {all * vol <= (size_t)10000000000 ? all : std::min(all, 4), std::min(all, 2)}) {
+        const size_t need = g * vol;
+        if (ctx->sgm_part.bytes >= need) return g;
+        if (need >= ctx->sgm_part_refused) continue;
+        if (ensure(ctx, ctx->sgm_part, need) == TDV_OK) return g;
+        ctx->sgm_part_refused = need;
+    }
+    return 0;
+}
+
 tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
                    const tdv_sgm_params* p, tdv_volume* aggreg, tdv_disparity* out, cudaStream_t st) {
     const int W = cost->width, H = cost->height, D = cost->depth;
     VolArg C = tdv::make_vol(*cost);
-    VolArg Sv;
-    if (aggreg) {
-        Sv = tdv::make_vol(*aggreg);
-    } else {
-        TDV_TRY(ensure(ctx, ctx->agg, (size_t)W * H * D * sizeof(float)));
-        tdv_volume tmp = *cost;
-        tmp.ptr = ctx->agg.ptr;
-        tmp.dtype = TDV_F32;  // the aggregation is float whatever the cost's type
-        Sv = tdv::make_vol(tmp);
-    }
     TDV_TRY(ensure_schedule(ctx, W, H, p->table, p->paths, st));
-    if (ctx->sched.defer_rows > 0)
-        TDV_TRY(ensure(ctx, ctx->defer, (size_t)ctx->sched.defer_rows * D * sizeof(float)));
     tdv::SgmArgs a;
-    a.defer = ctx->sched.defer_rows > 0 ? (float*)ctx->defer.ptr : nullptr;
+    a.defer = nullptr;
     a.C = C;
-    a.S = Sv;
     a.has_guide = guide ? 1 : 0;
     if (guide) a.guide = tdv::make_img(*guide);
     else memset(&a.guide, 0, sizeof(a.guide));
@@ -207,14 +216,37 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     a.p2 = p->p2;
     a.p2_adjust = p->p2_mode == TDV_P2_ADJUST;
     a.sem = p->semantics;
-    TDV_CUDA(tdv::launch_sgm_passes(a, ctx->sched, st, &ctx->timer));
+    const bool lr = out->lr_threshold >= 0 || out->disp_right;
+    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D) : 0;
+    const bool keep = aggreg || lr;  // the aggregated volume itself is needed
+    VolArg Sv;
+    if (aggreg) {
+        Sv = tdv::make_vol(*aggreg);
+    } else {
+        if (!group || keep || group < (int)ctx->sched.passes.size())
+            TDV_TRY(ensure(ctx, ctx->agg, (size_t)W * H * D * sizeof(float)));
+        tdv_volume tmp = *cost;
+        tmp.ptr = ctx->agg.ptr;
+        tmp.dtype = TDV_F32;  // the aggregation is float whatever the cost's type
+        Sv = tdv::make_vol(tmp);
+    }
+    a.S = Sv;
     uint16_t* disp = out->disp;
-    if (!disp && (out->lr_threshold >= 0 || out->disp_right)) {
+    if (!disp && lr) {
         TDV_TRY(ensure(ctx, ctx->misc, (size_t)W * H * sizeof(uint16_t)));
         disp = (uint16_t*)ctx->misc.ptr;
     }
-    TDV_CUDA(tdv::launch_wta(Sv, disp, out->disp_norm, st, &ctx->timer));
-    if (out->lr_threshold >= 0 || out->disp_right)
+    if (group) {
+        TDV_CUDA(tdv::launch_sgm_dirs(a, ctx->sched, (float*)ctx->sgm_part.ptr, group, (float*)Sv.ptr, keep, disp,
+                                      out->disp_norm, st, &ctx->timer));
+    } else {
+        if (ctx->sched.defer_rows > 0)
+            TDV_TRY(ensure(ctx, ctx->defer, (size_t)ctx->sched.defer_rows * D * sizeof(float)));
+        a.defer = ctx->sched.defer_rows > 0 ? (float*)ctx->defer.ptr : nullptr;
+        TDV_CUDA(tdv::launch_sgm_passes(a, ctx->sched, st, &ctx->timer));
+        TDV_CUDA(tdv::launch_wta(Sv, disp, out->disp_norm, st, &ctx->timer));
+    }
+    if (lr)
         TDV_CUDA(tdv::launch_lr(Sv, disp, out->disp_norm, out->disp_right,
                                 out->lr_threshold >= 0 ? out->lr_threshold : 0x7FFFFFFF, st,
                                 &ctx->timer));
@@ -487,7 +519,7 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
                      ctx->misc.ptr || ctx->sched_buf.ptr || ctx->err.ptr || ctx->soft.ptr ||
                      ctx->agg2.ptr || ctx->defer.ptr || ctx->side || ctx->fw_buf.ptr || ctx->fside.ptr ||
                      ctx->lane_main || ctx->planes_b.ptr || ctx->agg_b.ptr || ctx->agg2_b.ptr || ctx->fside_b.ptr ||
-                     ctx->dirs.ptr || ctx->dirs_b.ptr;
+                     ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr;
     if (any) {
         DeviceScope ds(ctx->device);
         cudaDeviceSynchronize();
@@ -512,6 +544,7 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
         release_buf(ctx, ctx->fside_b);
         release_buf(ctx, ctx->dirs);
         release_buf(ctx, ctx->dirs_b);
+        release_buf(ctx, ctx->sgm_part);
         if (ctx->lane_main) cudaStreamDestroy(ctx->lane_main);
         if (ctx->lane_side) cudaStreamDestroy(ctx->lane_side);
         for (cudaEvent_t e : {ctx->lane_fork, ctx->lane_join, ctx->lane_start, ctx->lane_done})
@@ -529,7 +562,7 @@ tdv_status tdv_ctx_set_allocator(tdv_ctx* ctx, tdv_alloc_fn alloc, tdv_free_fn r
     if ((alloc == nullptr) != (release == nullptr))
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator and release must be set together");
     if (ctx->agg.ptr || ctx->cost.ptr || ctx->planes.ptr || ctx->codes.ptr || ctx->misc.ptr ||
-        ctx->sched_buf.ptr || ctx->defer.ptr || ctx->dirs.ptr || ctx->dirs_b.ptr)
+        ctx->sched_buf.ptr || ctx->defer.ptr || ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr)
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator must be set before any scratch exists");
     ctx->alloc = alloc;
     ctx->release = release;

@@ -140,6 +140,31 @@ bool build_schedule(int W, int H, int table, int paths, PassSchedule& out) {
         out.walks.insert(out.walks.end(), p.walks.begin(), p.walks.end());
         out.passes.push_back(ps);
     }
+    // line counts: each walk must run from one image edge to the other, at
+    // most one (merged) walk per line and pass
+    out.nl = W + H - 1;
+    out.mult.assign(out.passes.size() * (size_t)out.nl, 0);
+    out.lines = out.plain = ok;
+    for (size_t p = 0; p < out.passes.size() && ok; p++) {
+        const Pass& ps = out.passes[p];
+        const int s = ps.dx * ps.dy;
+        for (size_t i = ps.first; i < ps.first + ps.count; i++) {
+            const Walk& w = out.walks[i];
+            const int line = ps.dy == 0 ? w.sy : (ps.dx == 0 ? w.sx : w.sx - s * w.sy + (s > 0 ? H - 1 : 0));
+            uint16_t& m = out.mult[p * out.nl + line];
+            if (inside(w.sx - ps.dx, w.sy - ps.dy) || inside(w.sx + w.len * ps.dx, w.sy + w.len * ps.dy) || m != 0 ||
+                w.mult > 65535)
+                out.lines = false;
+            m = (uint16_t)w.mult;
+            if (w.mult != 1) out.plain = false;
+        }
+        const size_t lines = ps.dy == 0 ? H : (ps.dx == 0 ? W : out.nl);
+        if (ps.count != lines) out.plain = false;
+    }
+    // the first pass writes S: it must take every cell
+    if (ok && (out.passes.empty() || out.passes[0].count != (out.passes[0].dy == 0 ? (size_t)H : (size_t)W) ||
+               out.passes[0].dx * out.passes[0].dy != 0))
+        out.lines = false;
     return ok;
 }
 

@@ -42,8 +42,16 @@ struct PassSchedule {
     std::vector<Walk> walks;         // host copy
     std::vector<int32_t> deferred;   // indices (into walks) of repeated walks, pass by pass
     long long defer_rows = 0;        // deferred-buffer rows one pass needs at most
+    // Line counts of the passes run side by side (kernels_sgm_dirs.cu): per
+    // pass, for each line of its direction (row, column, or x - s*y), how often
+    // a walk takes it; `lines` tells whether every walk is a whole line.
+    bool lines = false;
+    bool plain = false;              // every pass takes every line once
+    int nl = 0;
+    std::vector<uint16_t> mult;      // [pass][nl]
     Walk* d_walks = nullptr;         // device copies (ctx scratch)
     int32_t* d_deferred = nullptr;
+    uint16_t* d_mult = nullptr;
 };
 
 // Optional per-kernel timing.  Every kernel of one ABI call is bracketed by
@@ -191,6 +199,9 @@ struct tdv_ctx {
     // that later calls of that size go straight to the accumulating passes
     Buf dirs, dirs_b;
     size_t dirs_refused = (size_t)-1;
+    // general path with the passes side by side (kernels_sgm_dirs.cu)
+    Buf sgm_part;
+    size_t sgm_part_refused = (size_t)-1;
     cudaStream_t lane_main = nullptr, lane_side = nullptr;
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr, lane_start = nullptr, lane_done = nullptr;
 };
@@ -246,6 +257,13 @@ struct SgmArgs {
     int p2_adjust, sem;
     float* defer;  // path costs of the repeated walks of one pass (PassSchedule::defer_rows x D)
 };
+// The passes side by side in groups of `group` volumes (at most
+// kMaxSideBySide) at `part`, sgm_dirs_volume() bytes each: S is stored when
+// `keep` (and between groups), the winners always.  Needs sch.lines.
+constexpr int kMaxSideBySide = 8;
+size_t sgm_dirs_volume(int W, int H, int D);
+cudaError_t launch_sgm_dirs(const SgmArgs& a, const PassSchedule& sch, float* part, int group, float* S, bool keep,
+                            uint16_t* disp, float* disp_norm, cudaStream_t st, Timer* tm);
 cudaError_t launch_sgm_passes(const SgmArgs& a, const PassSchedule& sch, cudaStream_t st, Timer* tm);
 cudaError_t launch_wta(const VolArg& V, uint16_t* disp, float* disp_norm, cudaStream_t st, Timer* tm);
 cudaError_t launch_lr(const VolArg& S, uint16_t* dispL, float* disp_norm, uint16_t* dispR,

@@ -156,6 +156,12 @@ tdv_status tdv_dp_scanline(tdv_ctx* ctx, const tdv_volume* cost, tdv_disparity* 
 tdv_status tdv_fast_wta(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right,
                         int32_t max_disp, int32_t radius, tdv_disparity* out, tdv_stream stream);
 
+/* The same over the pre-filtered pair: tdv_cost_filtered (TDV_COST_SSD)
+ * followed by tdv_wta without the DSI between them, the chain DevStereoMatcher
+ * runs by default (tdvision/devstereomatcher.cpp:22-48); equal maps. */
+tdv_status tdv_fast_wta_filtered(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right, int32_t filter,
+                                 int32_t max_disp, int32_t radius, tdv_disparity* out, tdv_stream stream);
+
 /* Birchfield-Tomasi cost recomputed inside the aggregation, no cost DSI:
  * the role of SemiGlobalLabDevRun (tdvision/semiglobal_lab.cu:232-282) with
  * the reference's cost and recurrence.  Integer-domain inputs (u8, scale 1,

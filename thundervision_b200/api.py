@@ -234,6 +234,17 @@ class Context:
                                         radius, ctypes.byref(o), _stream()))
         return self._result(disp, dn, dr)
 
+    def fast_wta_filtered(self, left, right, max_disp, radius=3, scale=1.0, prefilter="gauss5", norm=False):
+        """``cost_filtered(kind="ssd")`` followed by ``wta`` without the DSI
+        between them (tdv_fast_wta_filtered); equal maps."""
+        H, W = left.shape
+        f = {"gauss5": L.FILTER_GAUSS5, "median7": L.FILTER_MEDIAN7}[prefilter]
+        li, ri = _image(left, scale), _image(right, scale)
+        o, disp, dn, dr = self._outputs(W, H, left.device, norm, False, None)
+        self.check(L.lib().tdv_fast_wta_filtered(self.handle, ctypes.byref(li), ctypes.byref(ri), f, max_disp,
+                                                 radius, ctypes.byref(o), _stream()))
+        return self._result(disp, dn, dr)
+
     # ---- image stages either side of the path ------------------------
     def to_gray(self, color):
         """(H, W, 3) uint8 -> (H, W) float32 grey in [0, 1] (channel 0 weighted

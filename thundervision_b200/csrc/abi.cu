@@ -877,9 +877,8 @@ tdv_status tdv_dp_scanline(tdv_ctx* ctx, const tdv_volume* cost, tdv_disparity* 
     return TDV_OK;
 }
 
-tdv_status tdv_fast_wta(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right, int32_t D,
-                        int32_t radius, tdv_disparity* out, tdv_stream stream) {
-    if (!ctx) return TDV_ERR_INVALID_ARG;
+static tdv_status check_fast_wta(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right, int32_t D,
+                                 int32_t radius, tdv_disparity* out) {
     TDV_TRY(check_image(ctx, left, "left"));
     TDV_TRY(check_image(ctx, right, "right"));
     TDV_TRY(check_out(ctx, out));
@@ -889,10 +888,43 @@ tdv_status tdv_fast_wta(tdv_ctx* ctx, const tdv_image* left, const tdv_image* ri
         return fail(ctx, TDV_ERR_UNSUPPORTED, "fast WTA has no left-right check");
     if (left->width != right->width || left->height != right->height)
         return fail(ctx, TDV_ERR_INVALID_ARG, "left and right images differ in size");
+    return TDV_OK;
+}
+
+tdv_status tdv_fast_wta(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right, int32_t D,
+                        int32_t radius, tdv_disparity* out, tdv_stream stream) {
+    if (!ctx) return TDV_ERR_INVALID_ARG;
+    TDV_TRY(check_fast_wta(ctx, left, right, D, radius, out));
     TDV_DEVICE_SCOPE(ctx);
     ctx->timer.begin(S(stream));
     TDV_CUDA(tdv::launch_fast_wta(tdv::make_img(*left), tdv::make_img(*right), D, radius, out->disp,
                                   out->disp_norm, S(stream), &ctx->timer));
+    return TDV_OK;
+}
+
+tdv_status tdv_fast_wta_filtered(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right, int32_t filter,
+                                 int32_t D, int32_t radius, tdv_disparity* out, tdv_stream stream) {
+    if (!ctx) return TDV_ERR_INVALID_ARG;
+    TDV_TRY(check_fast_wta(ctx, left, right, D, radius, out));
+    if (filter != TDV_FILTER_GAUSS5 && filter != TDV_FILTER_MEDIAN7)
+        return fail(ctx, TDV_ERR_INVALID_ARG, "bad filter kind %d", filter);
+    TDV_DEVICE_SCOPE(ctx);
+    ctx->timer.begin(S(stream));
+    const tdv::ImgArg L = tdv::make_img(*left), R = tdv::make_img(*right);
+    if (filter == TDV_FILTER_GAUSS5 && tdv::cost_banded_supported(TDV_COST_SSD, radius, D, true)) {
+        TDV_CUDA(tdv::launch_fast_wta_banded(L, R, D, radius, true, out->disp, out->disp_norm, S(stream)));
+        ctx->timer.mark("fast_wta_filtered");
+        return TDV_OK;
+    }
+    // filter into scratch, then over the filtered images
+    const size_t n = (size_t)left->width * left->height;
+    TDV_TRY(ensure(ctx, ctx->misc, 2 * n * sizeof(float)));
+    float* fl = (float*)ctx->misc.ptr;
+    TDV_CUDA(tdv::launch_prefilter(L, filter, fl, S(stream)));
+    TDV_CUDA(tdv::launch_prefilter(R, filter, fl + n, S(stream)));
+    const tdv::ImgArg FL{fl, left->width, left->height, left->width, 0, 1.0f};
+    const tdv::ImgArg FR{fl + n, right->width, right->height, right->width, 0, 1.0f};
+    TDV_CUDA(tdv::launch_fast_wta(FL, FR, D, radius, out->disp, out->disp_norm, S(stream), &ctx->timer));
     return TDV_OK;
 }
 

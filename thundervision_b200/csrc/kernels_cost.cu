@@ -1,7 +1,8 @@
 // Matching-cost DSI writers, banded: Birchfield-Tomasi (tdvision/birchfieldcost.cu:14-59),
 // window SSD (ssd.cu:15-50) and un-centred NCC (crosscorrelation.cu:11-49).
 //
-// One CTA owns a tile of kTX x kTY pixels and all D disparities of them.
+// One CTA owns a tile of kTX x TY pixels (TY 4 or 8, see tall_tiles) and all D
+// disparities of them.
 //   * Staging: the rows the tile's windows touch are read once, clamped to
 //     each image's own edges and multiplied by its scale exactly as the
 //     per-cell reference fetch does, into shared memory: raw bands for SSD /
@@ -18,13 +19,18 @@
 //     (SSD) or product (NCC) is formed once per column and then accumulated
 //     into every pixel whose window holds it -- in each pixel's own row-major
 //     tap order, so every cell is rounded exactly as the reference's loop
-//     rounds it.
+//     rounds it.  SSD and NCC do this on two pixels at once with packed
+//     FP32 pairs (add/sub/fma.rn.f32x2, each half rounded as the scalar
+//     operation): pixels p and p + P/2 of a thread share a register pair, and
+//     the bands are staged as the pairs that needs, (b[c], b[c + P/2]), so no
+//     pair is ever assembled in registers.
 //   * Stores: a warp writes the D-contiguous run of one pixel, a full
 //     128-byte line per instruction in either DSI layout.
 // Cells with x - d < 0 are +INF (the reference's range rule).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 
@@ -36,10 +42,9 @@ namespace tdv {
 namespace {
 
 constexpr int kTX = 64;           // tile width (pixels)
-constexpr int kTY = 4;            // tile height (rows)
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxBandBytes = 100 * 1024;
+constexpr int kMaxBandBytes = 220 * 1024;
 
 __device__ __forceinline__ float fetch(const ImgArg& im, int x, int y) {
     x = min(max(x, 0), im.W - 1);
@@ -52,40 +57,87 @@ __device__ __forceinline__ float fetch(const ImgArg& im, int x, int y) {
 struct Geom {
     int D, Dw, G;      // disparities; lanes per pixel group (8, 16 or 32); groups per warp
     int rbw;           // right-band width: columns x0-(D-1)-r .. x0+kTX-1+r
-    int lbw;           // left-band width: columns x0-r .. x0+kTX-1+r, padded to 4 floats
+    unsigned long long nz;  // (-0, -0), see mul2
 };
 
-__host__ __device__ constexpr int left_band_width(int r) { return kTX + ((2 * r + 3) & ~3); }
-
-// Shared-memory layout (floats) of one tile.
-template <int KIND, int R>
+// Shared-memory layout (floats) of one tile; HP: half the pixels of a thread
+// (SSD and NCC).  The left band is kept per run of 2 HP pixels, as HP + 2R
+// pairs (l[x + j], l[x + j + HP]); the right band as one pair (r[c],
+// r[c + HP]) per column.
+template <int KIND, int R, int HP, int TY_>
 struct Band {
-    static constexpr int kRows = kTY + 2 * R;
-    __host__ __device__ static int rband(const Geom& g) { return KIND == TDV_COST_BT ? 3 * kTX * kTY : kRows * g.lbw; }
+    static constexpr int TY = TY_;
+    static constexpr int kRows = TY + 2 * R;
+    static constexpr int kSeg = kTX / (2 * HP);            // runs per row
+    static constexpr int kJ = (HP + 2 * R + 1) & ~1;       // pairs per run, padded to 16 bytes
+    static constexpr int kLeft = kSeg * kJ * 2;            // floats of a left row
+    __host__ __device__ static int rband(const Geom&) { return KIND == TDV_COST_BT ? 3 * kTX * TY : kRows * kLeft; }
     // NCC window sums: LS per tile pixel, RS per (row, column x - d)
-    __host__ __device__ static int ls(const Geom& g) { return rband(g) + kRows * g.rbw; }
-    __host__ __device__ static int rs(const Geom& g) { return ls(g) + kTX * kTY; }
+    __host__ __device__ static int ls(const Geom& g) { return rband(g) + kRows * g.rbw * 2; }
+    __host__ __device__ static int rs(const Geom& g) { return ls(g) + kTX * TY; }
     __host__ __device__ static int floats(const Geom& g) {
-        if (KIND == TDV_COST_BT) return 3 * kTX * kTY + 3 * kTY * (kTX + g.D - 1);
-        if (KIND == TDV_COST_SSD) return kRows * g.lbw + kRows * g.rbw;
-        return kRows * g.lbw + kRows * g.rbw + kTX * kTY + kTY * (kTX + g.D - 1);
+        if (KIND == TDV_COST_BT) return 3 * kTX * TY + 3 * TY * (kTX + g.D - 1);
+        if (KIND == TDV_COST_SSD) return ls(g);
+        return rs(g) + TY * (kTX + g.D - 1);
     }
     // With the Gaussian fused: BT first builds filtered bands of the left
     // (kTX + 2 columns) and right (kTX + D + 1 columns) rows; every kind needs
     // the raw rows with a 2-pixel halo and their row pass as scratch.
     __host__ __device__ static int fl_band(const Geom& g) { return floats(g); }
-    __host__ __device__ static int fr_band(const Geom& g) { return fl_band(g) + kTY * (kTX + 2); }
-    __host__ __device__ static int widest(const Geom& g) {
-        return KIND == TDV_COST_BT ? kTX + g.D + 1 : (g.lbw > g.rbw ? g.lbw : g.rbw);
-    }
+    __host__ __device__ static int fr_band(const Geom& g) { return fl_band(g) + TY * (kTX + 2); }
+    __host__ __device__ static int widest(const Geom& g) { return KIND == TDV_COST_BT ? kTX + g.D + 1 : g.rbw; }
     __host__ __device__ static int scratch(const Geom& g) {
-        return KIND == TDV_COST_BT ? fr_band(g) + kTY * (kTX + g.D + 1) : floats(g);
+        return KIND == TDV_COST_BT ? fr_band(g) + TY * (kTX + g.D + 1) : floats(g);
     }
     __host__ __device__ static int floats_filtered(const Geom& g) {
-        const int rows = (KIND == TDV_COST_BT ? kTY : kRows) + 4, w = widest(g);
+        const int rows = (KIND == TDV_COST_BT ? TY : kRows) + 4, w = widest(g);
         return scratch(g) + rows * (w + 4) + rows * w;
     }
+    // where column c (from the band's first) of a band row goes
+    static __device__ __forceinline__ void put_left(float* lrow, int c, float v) {
+#pragma unroll
+        for (int sgm = 0; sgm < kSeg; sgm++) {
+            const int j = c - 2 * HP * sgm;
+            if (j >= 0 && j < HP + 2 * R) lrow[(sgm * kJ + j) * 2] = v;
+            if (j >= HP && j < 2 * HP + 2 * R) lrow[(sgm * kJ + j - HP) * 2 + 1] = v;
+        }
+    }
+    static __device__ __forceinline__ void put_right(float* rrow, int c, float v) {
+        rrow[2 * c] = v;
+        if (c >= HP) rrow[2 * (c - HP) + 1] = v;
+    }
+    // left column c again
+    static __device__ __forceinline__ float left(const float* lrow, int c) {
+        int sgm = c / (2 * HP);
+        sgm = sgm < kSeg ? sgm : kSeg - 1;
+        const int j = c - 2 * HP * sgm;
+        return j < HP + 2 * R ? lrow[(sgm * kJ + j) * 2] : lrow[(sgm * kJ + j - HP) * 2 + 1];
+    }
 };
+
+// ------------------------------------------------------------ packed pairs
+using f2 = unsigned long long;  // two floats: pixel p in the low word, p + HP in the high
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a * b rounded on its own: a multiply-add of nz = (-0, -0), which leaves every
+// product, signed zeros included, as it is.  nz must not be a constant the
+// compiler sees: a packed product (or a multiply-add of a literal -0) is
+// contracted with the addition that follows it, explicit rounding or not.
+__device__ __forceinline__ f2 mul2(f2 a, f2 b, f2 nz) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+    return r;
+}
+__device__ __forceinline__ float lo2(f2 a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float hi2(f2 a) { return __uint_as_float((uint32_t)(a >> 32)); }
 
 // BT terms of one sample: I, min and max of {I, (I + I[-1]) / 2, (I + I[+1]) / 2}.
 __device__ __forceinline__ void bt_terms(const ImgArg& im, int x, int y, float& I, float& mi, float& ma) {
@@ -96,12 +148,12 @@ __device__ __forceinline__ void bt_terms(const ImgArg& im, int x, int y, float& 
     ma = fmaxf(a, fmaxf(b, I));
 }
 
-// band[row * bw + col] = G(clamp(c0 + col), clamp(r0 + row)) for the 5x5
+// put(row, col, G(clamp(c0 + col), clamp(r0 + row))) for the 5x5
 // Gaussian G of the image with replicated borders (the pre-filter kernel's
 // values, bit for bit): the raw rows the clamped range needs, with a 2-pixel
 // halo, then the row pass, then the column pass, in that kernel's order.
-__device__ void gauss_band(const ImgArg& im, int c0, int ncols, int r0, int nrows, float* band, int bw,
-                           float* scratch) {
+template <typename Put>
+__device__ void gauss_band(const ImgArg& im, int c0, int ncols, int r0, int nrows, Put put, float* scratch) {
     const int tid = threadIdx.x;
     const int c_lo = min(max(c0, 0), im.W - 1), c_hi = min(max(c0 + ncols - 1, 0), im.W - 1);
     const int r_lo = min(max(r0, 0), im.H - 1), r_hi = min(max(r0 + nrows - 1, 0), im.H - 1);
@@ -123,7 +175,7 @@ __device__ void gauss_band(const ImgArg& im, int c0, int ncols, int r0, int nrow
         const int row = i / ncols, col = i - row * ncols;
         const int cc = min(max(c0 + col, 0), im.W - 1) - c_lo, rr = min(max(r0 + row, 0), im.H - 1) - r_lo;
         const float* t = rp + rr * nc + cc;
-        band[row * bw + col] = gauss5(t[0], t[nc], t[2 * nc], t[3 * nc], t[4 * nc]);
+        put(row, col, gauss5(t[0], t[nc], t[2 * nc], t[3 * nc], t[4 * nc]));
     }
     __syncthreads();
 }
@@ -138,25 +190,25 @@ __device__ __forceinline__ void bt_terms_band(const float* b, float& I, float& m
     ma = fmaxf(a, fmaxf(c, I));
 }
 
-template <int R>
+template <int R, int HP, int TY>
 __device__ void ncc_sums(const Geom& g, float* sm);
 
-template <int KIND, int R>
+template <int KIND, int R, int HP, int TY>
 __device__ void stage_plain(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0, int y0, float* sm) {
-    using B = Band<KIND, R>;
+    using B = Band<KIND, R, HP, TY>;
     const int tid = threadIdx.x;
     if (KIND == TDV_COST_BT) {
-        float* lt = sm;                  // [3][kTY][kTX]
-        float* rt = sm + B::rband(g);    // [3][kTY][kTX + D - 1]
-        for (int i = tid; i < kTX * kTY; i += kThreads) {
+        float* lt = sm;                  // [3][B::TY][kTX]
+        float* rt = sm + B::rband(g);    // [3][B::TY][kTX + D - 1]
+        for (int i = tid; i < kTX * B::TY; i += kThreads) {
             const int row = i / kTX, col = i - row * kTX;
             float I, mi, ma;
             bt_terms(L, x0 + col, y0 + row, I, mi, ma);
             lt[i] = I;
-            lt[kTX * kTY + i] = mi;
-            lt[2 * kTX * kTY + i] = ma;
+            lt[kTX * B::TY + i] = mi;
+            lt[2 * kTX * B::TY + i] = ma;
         }
-        const int rw = kTX + g.D - 1, n = rw * kTY;
+        const int rw = kTX + g.D - 1, n = rw * B::TY;
         float2* rmm = reinterpret_cast<float2*>(rt + n);  // (min, max) pairs, 8-byte aligned
         for (int i = tid; i < n; i += kThreads) {
             const int row = i / rw, col = i - row * rw;
@@ -167,80 +219,85 @@ __device__ void stage_plain(const ImgArg& L, const ImgArg& Rim, const Geom& g, i
         }
         return;
     }
-    float* lb = sm;                       // [kRows][lbw], column x0 - R at index 0
-    float* rb = sm + B::rband(g);         // [kRows][rbw], column x0 - (D-1) - R at index 0
-    for (int i = tid; i < B::kRows * g.lbw; i += kThreads) {
-        const int row = i / g.lbw, col = i - row * g.lbw;
-        lb[i] = fetch(L, x0 - R + col, y0 - R + row);
+    // left columns x0 - R .. x0 + kTX - 1 + R, right columns x0 - (D-1) - R ..
+    constexpr int lw = kTX + 2 * R;
+    float* lb = sm;
+    float* rb = sm + B::rband(g);
+    for (int i = tid; i < B::kRows * lw; i += kThreads) {
+        const int row = i / lw, col = i - row * lw;
+        B::put_left(lb + row * B::kLeft, col, fetch(L, x0 - R + col, y0 - R + row));
     }
     for (int i = tid; i < B::kRows * g.rbw; i += kThreads) {
         const int row = i / g.rbw, col = i - row * g.rbw;
-        rb[i] = fetch(Rim, x0 - (g.D - 1) - R + col, y0 - R + row);
+        B::put_right(rb + row * g.rbw * 2, col, fetch(Rim, x0 - (g.D - 1) - R + col, y0 - R + row));
     }
     if (KIND != TDV_COST_NCC) return;
     __syncthreads();
-    ncc_sums<R>(g, sm);
+    ncc_sums<R, HP, TY>(g, sm);
 }
 
 // NCC: window sums of squares in the reference's tap order (rows, then
-// columns), LS per tile pixel from the left band, RS per column x - d.
-template <int R>
+// columns), LS per tile pixel from the left band, RS per column x - d, two
+// HP-apart pixels or columns at once.
+template <int R, int HP, int TY>
 __device__ void ncc_sums(const Geom& g, float* sm) {
-    using B = Band<TDV_COST_NCC, R>;
+    using B = Band<TDV_COST_NCC, R, HP, TY>;
     const int tid = threadIdx.x;
-    const float* lb = sm;
-    const float* rb = sm + B::rband(g);
+    const f2* lb = reinterpret_cast<const f2*>(sm);
+    const f2* rb = reinterpret_cast<const f2*>(sm + B::rband(g));
     float* ls = sm + B::ls(g);
     float* rs = sm + B::rs(g);
-    for (int i = tid; i < kTX * kTY; i += kThreads) {
-        const int row = i / kTX, col = i - row * kTX;
-        float s = 0.0f;
-        for (int a = 0; a <= 2 * R; a++)
-            for (int b = 0; b <= 2 * R; b++) {
-                const float v = lb[(row + a) * g.lbw + col + b];
-                s = __fadd_rn(s, __fmul_rn(v, v));
-            }
-        ls[i] = s;
+    auto window = [&](const f2* p, int stride) {
+        f2 s = 0ull;
+#pragma unroll 1
+        for (int a = 0; a <= 2 * R; a++, p += stride)
+#pragma unroll
+            for (int b = 0; b <= 2 * R; b++) s = add2(s, mul2(p[b], p[b], g.nz));
+        return s;
+    };
+    for (int i = tid; i < B::TY * kTX / 2; i += kThreads) {
+        const int row = i / (kTX / 2), q = i - row * (kTX / 2), run = q / HP, j = q - run * HP;
+        const f2 s = window(lb + row * (B::kLeft / 2) + run * B::kJ + j, B::kLeft / 2);
+        ls[row * kTX + run * 2 * HP + j] = lo2(s);
+        ls[row * kTX + run * 2 * HP + j + HP] = hi2(s);
     }
-    const int rw = kTX + g.D - 1;
-    for (int i = tid; i < rw * kTY; i += kThreads) {
-        const int row = i / rw, col = i - row * rw;
-        float s = 0.0f;
-        for (int a = 0; a <= 2 * R; a++)
-            for (int b = 0; b <= 2 * R; b++) {
-                const float v = rb[(row + a) * g.rbw + col + b];
-                s = __fadd_rn(s, __fmul_rn(v, v));
-            }
-        rs[i] = s;
+    const int rw = kTX + g.D - 1, half = (rw + 2 * HP - 1) / (2 * HP) * HP;
+    for (int i = tid; i < half * B::TY; i += kThreads) {
+        const int row = i / half, q = i - row * half, c = q / HP * 2 * HP + q % HP;
+        if (c >= rw) continue;
+        const f2 s = window(rb + row * g.rbw + c, g.rbw);
+        rs[row * rw + c] = lo2(s);
+        if (c + HP < rw) rs[row * rw + c + HP] = hi2(s);
     }
 }
 
 // Fills the tile's bands (and, when FILT, writes the filtered left samples of
 // the tile's own pixels to fl_out, W x H dense).
-template <int KIND, int R, bool FILT>
+template <int KIND, int R, int HP, bool FILT, int TY>
 __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0, int y0, float* sm, int W, int H,
                       float* fl_out) {
-    using B = Band<KIND, R>;
+    using B = Band<KIND, R, HP, TY>;
     const int tid = threadIdx.x;
     if (FILT && KIND == TDV_COST_BT) {
-        float* fl = sm + B::fl_band(g);     // [kTY][kTX + 2]: columns x0 - 1 .. x0 + kTX
-        float* fr = sm + B::fr_band(g);     // [kTY][kTX + D + 1]: columns x0 - D .. x0 + kTX
+        float* fl = sm + B::fl_band(g);     // [B::TY][kTX + 2]: columns x0 - 1 .. x0 + kTX
+        float* fr = sm + B::fr_band(g);     // [B::TY][kTX + D + 1]: columns x0 - D .. x0 + kTX
         float* scr = sm + B::scratch(g);
-        gauss_band(L, x0 - 1, kTX + 2, y0, kTY, fl, kTX + 2, scr);
-        gauss_band(Rim, x0 - g.D, kTX + g.D + 1, y0, kTY, fr, kTX + g.D + 1, scr);
+        gauss_band(L, x0 - 1, kTX + 2, y0, B::TY, [&](int r, int c, float v) { fl[r * (kTX + 2) + c] = v; }, scr);
+        gauss_band(Rim, x0 - g.D, kTX + g.D + 1, y0, B::TY,
+                   [&](int r, int c, float v) { fr[r * (kTX + g.D + 1) + c] = v; }, scr);
         float* lt = sm;
         float* rt = sm + B::rband(g);
-        for (int i = tid; i < kTX * kTY; i += kThreads) {
+        for (int i = tid; i < kTX * B::TY; i += kThreads) {
             const int row = i / kTX, col = i - row * kTX;
             float I, mi, ma;
             bt_terms_band(fl + row * (kTX + 2) + col, I, mi, ma);
             lt[i] = I;
-            lt[kTX * kTY + i] = mi;
-            lt[2 * kTX * kTY + i] = ma;
+            lt[kTX * B::TY + i] = mi;
+            lt[2 * kTX * B::TY + i] = ma;
             const int x = x0 + col, y = y0 + row;
             if (fl_out && x < W && y < H) fl_out[(size_t)y * W + x] = I;
         }
-        const int rw = kTX + g.D - 1, n = rw * kTY;
+        const int rw = kTX + g.D - 1, n = rw * B::TY;
         float2* rmm = reinterpret_cast<float2*>(rt + n);
         for (int i = tid; i < n; i += kThreads) {
             const int row = i / rw, col = i - row * rw;
@@ -255,27 +312,89 @@ __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0,
         float* lb = sm;
         float* rb = sm + B::rband(g);
         float* scr = sm + B::scratch(g);
-        gauss_band(L, x0 - R, g.lbw, y0 - R, B::kRows, lb, g.lbw, scr);
-        gauss_band(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows, rb, g.rbw, scr);
+        gauss_band(L, x0 - R, kTX + 2 * R, y0 - R, B::kRows,
+                   [&](int r, int c, float v) { B::put_left(lb + r * B::kLeft, c, v); }, scr);
+        gauss_band(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows,
+                   [&](int r, int c, float v) { B::put_right(rb + r * g.rbw * 2, c, v); }, scr);
         if (fl_out)
-            for (int i = tid; i < kTX * kTY; i += kThreads) {
+            for (int i = tid; i < kTX * B::TY; i += kThreads) {
                 const int row = i / kTX, col = i - row * kTX;
                 const int x = x0 + col, y = y0 + row;
-                if (x < W && y < H) fl_out[(size_t)y * W + x] = lb[(row + R) * g.lbw + col + R];
+                if (x < W && y < H) fl_out[(size_t)y * W + x] = B::left(lb + (row + R) * B::kLeft, col + R);
             }
-        if (KIND == TDV_COST_NCC) ncc_sums<R>(g, sm);
+        if (KIND == TDV_COST_NCC) ncc_sums<R, HP, TY>(g, sm);
         return;
     }
-    stage_plain<KIND, R>(L, Rim, g, x0, y0, sm);
+    stage_plain<KIND, R, HP, TY>(L, Rim, g, x0, y0, sm);
 }
 
-template <int KIND, int R, int P, bool FILT>
+// Window sums of one disparity over 2 HP pixels of two adjacent rows: SSD, or
+// the NCC's numerator; acc[i] for row i.  l: the run's left pairs in the first
+// row's window; r: the right pairs from column x - d - R of that row on.
+//
+// What bounds it: FP32.  A 16-pixel, 7x7 window row is 22 differences, 22
+// squares and 112 sums; one by one with 28 loads that was 184 instructions per
+// output row and window row (91 % of the issue slots).  As pairs it is 28 + 56
+// at the packed rate (0.93 scalar operations a clock and scheduler, against
+// 0.69 unpacked) and 21 loads; a row of taps serves both output rows (each
+// still adds its own window's rows in order), which leaves 16 + 56 and 12.
+// DSI writer, D = 64, ms before / pairs / pairs and two rows: 1920x1080 SSD 7x7
+// 0.456 / 0.396 / 0.319, NCC 9x9 0.732 / 0.669 / 0.603; 640x480 SSD 5x5 0.056 /
+// 0.049 / 0.040, NCC 9x9 0.127 / 0.119 / 0.110.
+template <int KIND, int R, int HP>
+__device__ __forceinline__ void window_sums(const f2* l, int lstride, const f2* r, int rstride, f2 nz,
+                                            f2 (*acc)[HP]) {
+    constexpr int NJ = HP + 2 * R;
+    constexpr int NJ2 = (NJ + 1) & ~1;
+    f2 t[NJ];
+    auto taps = [&]() {
+        f2 lw[NJ2];
+#pragma unroll
+        for (int q = 0; q < NJ2 / 2; q++) {
+            const ulonglong2 v = reinterpret_cast<const ulonglong2*>(l)[q];  // the same for every lane
+            lw[2 * q] = v.x;
+            lw[2 * q + 1] = v.y;
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; j++) {
+            if (KIND == TDV_COST_SSD) {
+                const f2 df = sub2(lw[j], r[j]);
+                t[j] = mul2(df, df, nz);
+            } else {
+                t[j] = mul2(lw[j], r[j], nz);
+            }
+        }
+        l += lstride;
+        r += rstride;
+    };
+    auto add_row = [&](f2* s) {
+#pragma unroll
+        for (int b = 0; b <= 2 * R; b++)
+#pragma unroll
+            for (int p = 0; p < HP; p++) s[p] = add2(s[p], t[p + b]);
+    };
+#pragma unroll
+    for (int p = 0; p < HP; p++) acc[0][p] = acc[1][p] = 0ull;
+    taps();
+    add_row(acc[0]);
+#pragma unroll 1
+    for (int a = 1; a <= 2 * R; a++) {
+        taps();
+        add_row(acc[0]);
+        add_row(acc[1]);
+    }
+    taps();
+    add_row(acc[1]);
+}
+
+template <int KIND, int R, int P, bool FILT, int TY>
 __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Rim, VolArg out, Geom g,
                                                              int tiles_x, float* fl_out) {
     extern __shared__ __align__(16) float sm[];
-    using B = Band<KIND, R>;
-    const int x0 = (blockIdx.x % tiles_x) * kTX, y0 = (blockIdx.x / tiles_x) * kTY;
-    stage<KIND, R, FILT>(L, Rim, g, x0, y0, sm, out.W, out.H, fl_out);
+    constexpr int HP = P / 2;
+    using B = Band<KIND, R, HP, TY>;
+    const int x0 = (blockIdx.x % tiles_x) * kTX, y0 = (blockIdx.x / tiles_x) * B::TY;
+    stage<KIND, R, HP, FILT, TY>(L, Rim, g, x0, y0, sm, out.W, out.H, fl_out);
     __syncthreads();
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -284,7 +403,7 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
     const int span = P * g.G;                   // pixels of one work item
     const int groups = kTX / span;
     const int chunks = (D + g.Dw - 1) / g.Dw;
-    const int items = kTY * groups * chunks;
+    const int items = B::TY / 2 * groups * chunks;  // (SSD, NCC) two rows each
     float* const outp = (float*)out.ptr;
 
     if (KIND == TDV_COST_BT) {
@@ -292,8 +411,8 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
         // so each pixel's left terms are read from shared memory once
         const float* lt = sm;
         const float* rt = sm + B::rband(g);
-        const int n = (kTX + D - 1) * kTY;
-        for (int it = warp; it < kTY * groups; it += kWarps) {
+        const int n = (kTX + D - 1) * B::TY;
+        for (int it = warp; it < B::TY * groups; it += kWarps) {
             const int grp = it % groups, row = it / groups;
             const int y = y0 + row;
             const int xs = x0 + grp * span + sub * P;
@@ -302,8 +421,8 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
             for (int p = 0; p < P; p++) {
                 const int li = row * kTX + (xs + p - x0);
                 lI[p] = lt[li];
-                lImi[p] = lt[kTX * kTY + li];
-                lIma[p] = lt[2 * kTX * kTY + li];
+                lImi[p] = lt[kTX * B::TY + li];
+                lIma[p] = lt[2 * kTX * B::TY + li];
             }
             const float2* rmm = reinterpret_cast<const float2*>(rt + n);
             const bool rows_in = y < H && xs + P <= W;
@@ -359,68 +478,47 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
         for (int it = warp; it < items; it += kWarps) {
             const int chunk = it % chunks;
             const int rest = it / chunks;
-            const int grp = rest % groups, row = rest / groups;
-            const int y = y0 + row;
+            const int grp = rest % groups, row = 2 * (rest / groups);
             const int xs = x0 + grp * span + sub * P;   // first pixel of this thread
             const int d = chunk * g.Dw + dl;
             const bool dok = d < D;
             const int de = dok ? d : D - 1;             // lanes past D read in-band columns, store nothing
-            float v[P];
-            {
-                constexpr int NJ = P + 2 * R;
-                float acc[P];
-    #pragma unroll
-                for (int p = 0; p < P; p++) acc[p] = 0.0f;
-                const float* lb = sm + (size_t)row * g.lbw + (xs - x0);
-                const float* rb = sm + B::rband(g) + (size_t)row * g.rbw + (xs - de) - (x0 - (D - 1));
-                constexpr int NJ4 = (NJ + 3) & ~3;
-    #pragma unroll 1
-                for (int a = 0; a <= 2 * R; a++) {
-                    // the left window is the same for every lane: 128-bit
-                    // broadcast reads (the row start is a multiple of 16 floats
-                    // into a row padded to 4)
-                    float lw[NJ4];
-                    const float4* l4 = reinterpret_cast<const float4*>(lb + a * g.lbw);
-    #pragma unroll
-                    for (int q = 0; q < NJ4 / 4; q++) {
-                        const float4 f = l4[q];
-                        lw[4 * q] = f.x;
-                        lw[4 * q + 1] = f.y;
-                        lw[4 * q + 2] = f.z;
-                        lw[4 * q + 3] = f.w;
-                    }
-                    float t[NJ];
-    #pragma unroll
-                    for (int j = 0; j < NJ; j++) {
-                        const float lv = lw[j], rv = rb[a * g.rbw + j];
-                        if (KIND == TDV_COST_SSD) {
-                            const float df = __fsub_rn(lv, rv);
-                            t[j] = __fmul_rn(df, df);
-                        } else {
-                            t[j] = __fmul_rn(lv, rv);
-                        }
-                    }
-    #pragma unroll
-                    for (int b = 0; b <= 2 * R; b++)
-    #pragma unroll
-                        for (int p = 0; p < P; p++) acc[p] = __fadd_rn(acc[p], t[p + b]);
+            f2 acc[2][HP];
+            window_sums<KIND, R, HP>(
+                reinterpret_cast<const f2*>(sm) + row * (B::kLeft / 2) + (xs - x0) / P * B::kJ, B::kLeft / 2,
+                reinterpret_cast<const f2*>(sm + B::rband(g)) + row * g.rbw + (xs - de) - (x0 - (D - 1)), g.rbw, g.nz,
+                acc);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int y = y0 + row + i;
+                float v[P];
+#pragma unroll
+                for (int p = 0; p < HP; p++) {
+                    v[p] = lo2(acc[i][p]);
+                    v[p + HP] = hi2(acc[i][p]);
                 }
-                if (KIND == TDV_COST_SSD) {
-    #pragma unroll
-                    for (int p = 0; p < P; p++) v[p] = acc[p];
-                } else {
-                    const float* ls = sm + B::ls(g) + row * kTX + (xs - x0);
-                    const float* rs = sm + B::rs(g) + row * (kTX + D - 1) + (xs - de) - (x0 - (D - 1));
-    #pragma unroll
+                if (KIND == TDV_COST_NCC) {
+                    const float* ls = sm + B::ls(g) + (row + i) * kTX + (xs - x0);
+                    const float* rs = sm + B::rs(g) + (row + i) * (kTX + D - 1) + (xs - de) - (x0 - (D - 1));
+#pragma unroll
                     for (int p = 0; p < P; p++)
-                        v[p] = __fsub_rn(1.0f, __fdiv_rn(acc[p], __fsqrt_rn(__fmul_rn(ls[p], rs[p]))));
+                        v[p] = __fsub_rn(1.0f, __fdiv_rn(v[p], __fsqrt_rn(__fmul_rn(ls[p], rs[p]))));
                 }
-            }
-            if (!dok || y >= H) continue;
-    #pragma unroll
-            for (int p = 0; p < P; p++) {
-                const int x = xs + p;
-                if (x < W) outp[x * out.sx + y * out.sy + d] = (x - d < 0) ? CUDART_INF_F : v[p];
+                if (!dok || y >= H) continue;
+                float* op = outp + (xs * out.sx + y * out.sy + d);
+                if (xs + P <= W && xs - d >= 0) {  // every cell in the image and in range
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        *op = v[p];
+                        op += out.sx;
+                    }
+                } else {
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        const int x = xs + p;
+                        if (x < W) op[p * out.sx] = (x - d < 0) ? CUDART_INF_F : v[p];
+                    }
+                }
             }
         }
     }
@@ -450,151 +548,151 @@ cudaError_t opt_in_once(Kern k, std::atomic<unsigned long long>& opted) {
 __device__ __forceinline__ uint32_t ssd_key(float v) { return min(__float_as_uint(v), 0x7F800000u); }
 
 // FastWTA (tdvision/fastwta.cu:32-53): the window SSD of the banded kernel
-// with the argmin over d fused in, no DSI.  A lane keeps the best (key, d)
-// of its own disparities over the chunks (strict <, so its lowest d wins a
-// tie), then the lanes of a pixel group merge by (key, d) -- the lowest d
-// among the smallest costs, d = 0 when no cost is finite, as the reference's
-// scan gives.  Eight pixels per thread (half the SSD kernel's sixteen) keep
-// the per-pixel best keys within a register budget that fits four blocks per
-// SM.
-template <int R, int P>
-__global__ void __launch_bounds__(kThreads) fastwta_band_kernel(ImgArg L, ImgArg Rim, int W, int H, Geom g,
+// with the argmin over d fused in, no DSI.  After each chunk of DW disparities
+// the lanes of a pixel group reduce every pixel's key and take the lowest d
+// holding it (d = 0 when no cost is finite, as the reference's scan gives; a
+// later chunk wins only with a smaller key).  The bests of a group's 2 x P
+// pixels are spread over its lanes, 2 P / DW each: kept per pixel in every
+// lane they took 122 registers and two blocks per SM.  1920x1080, D = 64, 7x7:
+// 0.50 ms -> 0.36; with the Gaussian fused 0.41, against 0.37 for the filtered
+// DSI and 0.13 for its winner.
+template <int R, int P, int DW, bool FILT, int TY>
+__global__ void __launch_bounds__(kThreads, 3) fastwta_band_kernel(ImgArg L, ImgArg Rim, int W, int H, Geom g,
                                                                 int tiles_x, uint16_t* disp, float* disp_norm) {
     extern __shared__ __align__(16) float sm[];
-    using B = Band<TDV_COST_SSD, R>;
-    const int x0 = (blockIdx.x % tiles_x) * kTX, y0 = (blockIdx.x / tiles_x) * kTY;
-    stage<TDV_COST_SSD, R, false>(L, Rim, g, x0, y0, sm, W, H, nullptr);
+    constexpr int HP = P / 2;
+    using B = Band<TDV_COST_SSD, R, HP, TY>;
+    const int x0 = (blockIdx.x % tiles_x) * kTX, y0 = (blockIdx.x / tiles_x) * B::TY;
+    stage<TDV_COST_SSD, R, HP, FILT, TY>(L, Rim, g, x0, y0, sm, W, H, nullptr);
     __syncthreads();
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int D = g.D;
-    const int sub = lane / g.Dw, dl = lane - sub * g.Dw;
-    const int span = P * g.G;
-    const int groups = kTX / span;
-    const int chunks = (D + g.Dw - 1) / g.Dw;
-    constexpr int NJ = P + 2 * R;
-    constexpr int NJ4 = (NJ + 3) & ~3;
+    const int sub = lane / DW, dl = lane % DW;
+    constexpr int span = P * (32 / DW);
+    constexpr int groups = kTX / span;
+    constexpr int NB = 2 * P / DW;  // pixels a lane keeps
+    const int chunks = (D + DW - 1) / DW;
 
-    for (int it = warp; it < kTY * groups; it += kWarps) {
-        const int grp = it % groups, row = it / groups;
-        const int y = y0 + row;
+    for (int it = warp; it < B::TY / 2 * groups; it += kWarps) {
+        const int grp = it % groups, row = 2 * (it / groups);
         const int xs = x0 + grp * span + sub * P;
-        uint32_t bk[P];
-        int bd[P];
+        uint32_t bk[NB];
+        int bd[NB];
 #pragma unroll
-        for (int p = 0; p < P; p++) {
-            bk[p] = 0xFFFFFFFFu;
-            bd[p] = dl;
+        for (int n = 0; n < NB; n++) {
+            bk[n] = 0xFFFFFFFFu;
+            bd[n] = 0;
         }
         for (int chunk = 0; chunk < chunks; chunk++) {
-            const int d = chunk * g.Dw + dl;
+            const int d = chunk * DW + dl;
             const bool dok = d < D;
             const int de = dok ? d : D - 1;
-            float acc[P];
+            f2 sums[2][HP];
+            window_sums<TDV_COST_SSD, R, HP>(
+                reinterpret_cast<const f2*>(sm) + row * (B::kLeft / 2) + (xs - x0) / P * B::kJ, B::kLeft / 2,
+                reinterpret_cast<const f2*>(sm + B::rband(g)) + row * g.rbw + (xs - de) - (x0 - (D - 1)), g.rbw, g.nz,
+                sums);
+            const int xin = dok ? d - xs : P;  // pixels p >= xin are in range
 #pragma unroll
-            for (int p = 0; p < P; p++) acc[p] = 0.0f;
-            const float* lb = sm + (size_t)row * g.lbw + (xs - x0);
-            const float* rb = sm + B::rband(g) + (size_t)row * g.rbw + (xs - de) - (x0 - (D - 1));
-#pragma unroll 1
-            for (int a = 0; a <= 2 * R; a++) {
-                float lw[NJ4];
-                const float4* l4 = reinterpret_cast<const float4*>(lb + a * g.lbw);
-#pragma unroll
-                for (int q = 0; q < NJ4 / 4; q++) {
-                    const float4 f = l4[q];
-                    lw[4 * q] = f.x;
-                    lw[4 * q + 1] = f.y;
-                    lw[4 * q + 2] = f.z;
-                    lw[4 * q + 3] = f.w;
-                }
-                float t[NJ];
-#pragma unroll
-                for (int j = 0; j < NJ; j++) {
-                    const float df = __fsub_rn(lw[j], rb[a * g.rbw + j]);
-                    t[j] = __fmul_rn(df, df);
-                }
-#pragma unroll
-                for (int b = 0; b <= 2 * R; b++)
-#pragma unroll
-                    for (int p = 0; p < P; p++) acc[p] = __fadd_rn(acc[p], t[p + b]);
-            }
-            if (dok && xs - d >= 0) {  // every cell of the chunk in range
+            for (int i = 0; i < 2; i++)
 #pragma unroll
                 for (int p = 0; p < P; p++) {
-                    const uint32_t key = ssd_key(acc[p]);
-                    if (key < bk[p]) {
-                        bk[p] = key;
-                        bd[p] = d;
-                    }
-                }
-            } else if (dok) {
+                    const uint32_t mine =
+                        p >= xin ? ssd_key(p < HP ? lo2(sums[i][p]) : hi2(sums[i][p - HP])) : 0xFFFFFFFFu;
+                    uint32_t k = mine;
+                    uint32_t dd;
+                    if (DW == 32) {
+                        k = __reduce_min_sync(0xFFFFFFFFu, k);
+                        dd = __reduce_min_sync(0xFFFFFFFFu, mine == k ? (uint32_t)d : 0x7FFFFFFFu);
+                    } else {
 #pragma unroll
-                for (int p = 0; p < P; p++) {
-                    const uint32_t key = ssd_key(acc[p]);
-                    if (xs + p - d >= 0 && key < bk[p]) {
-                        bk[p] = key;
-                        bd[p] = d;
+                        for (int off = DW >> 1; off > 0; off >>= 1)
+                            k = min(k, __shfl_xor_sync(0xFFFFFFFFu, k, off));
+                        dd = mine == k ? (uint32_t)d : 0x7FFFFFFFu;
+#pragma unroll
+                        for (int off = DW >> 1; off > 0; off >>= 1)
+                            dd = min(dd, __shfl_xor_sync(0xFFFFFFFFu, dd, off));
+                    }
+                    const int idx = i * P + p;
+                    if (dl == idx % DW && k < bk[idx / DW]) {
+                        bk[idx / DW] = k;
+                        bd[idx / DW] = (int)dd;
                     }
                 }
-            }
         }
 #pragma unroll
-        for (int p = 0; p < P; p++) {
-            uint32_t k = bk[p];
-            int dd = bd[p];
-            if (g.Dw == 32) {
-                // the warp is one pixel group: the smallest key, then the
-                // lowest d among the lanes holding it
-                k = __reduce_min_sync(0xFFFFFFFFu, k);
-                dd = (int)__reduce_min_sync(0xFFFFFFFFu, bk[p] == k ? (unsigned)dd : 0x7FFFFFFFu);
-            } else {
-                for (int off = g.Dw >> 1; off > 0; off >>= 1) {
-                    const uint32_t ok = __shfl_xor_sync(0xFFFFFFFFu, k, off);
-                    const int od = __shfl_xor_sync(0xFFFFFFFFu, dd, off);
-                    if (ok < k || (ok == k && od < dd)) {
-                        k = ok;
-                        dd = od;
-                    }
-                }
-            }
-            const int x = xs + p;
-            if (dl == 0 && x < W && y < H) {
+        for (int n = 0; n < NB; n++) {
+            const int idx = n * DW + dl, i = idx / P, p = idx - i * P;
+            const int x = xs + p, y = y0 + row + i;
+            if (x < W && y < H) {
                 const size_t o = (size_t)y * W + x;
-                if (disp) disp[o] = (uint16_t)dd;
-                if (disp_norm) disp_norm[o] = __fdiv_rn((float)dd, (float)D);
+                if (disp) disp[o] = (uint16_t)bd[n];
+                if (disp_norm) disp_norm[o] = __fdiv_rn((float)bd[n], (float)D);
             }
         }
     }
 }
 
-template <int R>
-cudaError_t launch_fastwta_r(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
-                             cudaStream_t st) {
-    const int bytes = Band<TDV_COST_SSD, R>::floats(g) * 4;
-    auto k = fastwta_band_kernel<R, 8>;
+// Tile height: 8 rows share a window's halo, its filter and its window sums
+// better, 4 spread a small image over the chip (NCC 9x9, D = 64: 0.603 / 0.620
+// ms at 1920x1080, 0.120 / 0.110 at 640x480; BT 0.125 / 0.132 and 0.029 /
+// 0.025): 8 from ten rounds of tiles over 148 SMs on.
+bool tall_tiles(int W, int H) { return (long long)((W + kTX - 1) / kTX) * ((H + 7) / 8) >= 1480; }
+
+template <int R, int DW, bool FILT, int TY>
+cudaError_t launch_fastwta_ty(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
+                              cudaStream_t st) {
+    constexpr int P = 16;
+    using B = Band<TDV_COST_SSD, R, P / 2, TY>;
+    const int bytes = (FILT ? B::floats_filtered(g) : B::floats(g)) * 4;
+    auto k = fastwta_band_kernel<R, P, DW, FILT, TY>;
     static std::atomic<unsigned long long> opted{0};
     if (bytes > 48 * 1024) {
         const cudaError_t e = opt_in_once(k, opted);
         if (e != cudaSuccess) return e;
     }
-    const int tiles_x = (L.W + kTX - 1) / kTX, tiles_y = (L.H + kTY - 1) / kTY;
+    const int tiles_x = (L.W + kTX - 1) / kTX, tiles_y = (L.H + TY - 1) / TY;
     k<<<tiles_x * tiles_y, kThreads, bytes, st>>>(L, Rim, L.W, L.H, g, tiles_x, disp, disp_norm);
+    return cudaGetLastError();
+}
+
+template <int R, int DW, bool FILT>
+cudaError_t launch_fastwta_dw(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
+                              cudaStream_t st) {
+    return tall_tiles(L.W, L.H) ? launch_fastwta_ty<R, DW, FILT, 8>(L, Rim, g, disp, disp_norm, st)
+                                : launch_fastwta_ty<R, DW, FILT, 4>(L, Rim, g, disp, disp_norm, st);
+}
+
+template <int R, bool FILT>
+cudaError_t launch_fastwta_r(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
+                             cudaStream_t st) {
+    if (g.Dw == 32) return launch_fastwta_dw<R, 32, FILT>(L, Rim, g, disp, disp_norm, st);
+    if (g.Dw == 16) return launch_fastwta_dw<R, 16, FILT>(L, Rim, g, disp, disp_norm, st);
+    return launch_fastwta_dw<R, 8, FILT>(L, Rim, g, disp, disp_norm, st);
+}
+
+template <int KIND, int R, int P, bool FILT, int TY>
+cudaError_t launch_ty(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
+                      cudaStream_t st) {
+    using B = Band<KIND, R, P / 2, TY>;
+    const int bytes = (FILT ? B::floats_filtered(g) : B::floats(g)) * 4;
+    auto k = cost_band_kernel<KIND, R, P, FILT, TY>;
+    static std::atomic<unsigned long long> opted{0};
+    if (bytes > 48 * 1024) {
+        const cudaError_t e = opt_in_once(k, opted);
+        if (e != cudaSuccess) return e;
+    }
+    const int tiles_x = (out.W + kTX - 1) / kTX, tiles_y = (out.H + TY - 1) / TY;
+    k<<<tiles_x * tiles_y, kThreads, bytes, st>>>(L, Rim, out, g, tiles_x, fl_out);
     return cudaGetLastError();
 }
 
 template <int KIND, int R, int P, bool FILT>
 cudaError_t launch_one(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
                        cudaStream_t st) {
-    const int bytes = (FILT ? Band<KIND, R>::floats_filtered(g) : Band<KIND, R>::floats(g)) * 4;
-    auto k = cost_band_kernel<KIND, R, P, FILT>;
-    static std::atomic<unsigned long long> opted{0};
-    if (bytes > 48 * 1024) {
-        const cudaError_t e = opt_in_once(k, opted);
-        if (e != cudaSuccess) return e;
-    }
-    const int tiles_x = (out.W + kTX - 1) / kTX, tiles_y = (out.H + kTY - 1) / kTY;
-    k<<<tiles_x * tiles_y, kThreads, bytes, st>>>(L, Rim, out, g, tiles_x, fl_out);
-    return cudaGetLastError();
+    return tall_tiles(out.W, out.H) ? launch_ty<KIND, R, P, FILT, 8>(L, Rim, out, g, fl_out, st)
+                                    : launch_ty<KIND, R, P, FILT, 4>(L, Rim, out, g, fl_out, st);
 }
 
 template <int KIND, bool FILT>
@@ -608,24 +706,32 @@ cudaError_t dispatch_r(int r, const ImgArg& L, const ImgArg& Rim, const VolArg& 
     }
 }
 
+template <int KIND, int R>
+long long band_floats_r(const Geom& g, bool filt) {
+    using B = Band<KIND, R, KIND == TDV_COST_BT ? 4 : 8, 8>;  // the taller tile's
+    return filt ? B::floats_filtered(g) : B::floats(g);
+}
+
+Geom geom(int r, int D) {
+    Geom g;
+    g.D = D;
+    g.Dw = D >= 32 ? 32 : D > 8 ? 16 : 8;
+    g.G = 32 / g.Dw;
+    g.rbw = kTX + D - 1 + 2 * r;
+    g.nz = 0x8000000080000000ull;
+    return g;
+}
+
 long long band_floats(int kind, int r, int D, bool filt) {
-    const long long lbw = left_band_width(r), rbw = kTX + D - 1 + 2 * r;
-    long long f;
-    if (kind == TDV_COST_BT) {
-        f = 3LL * kTX * kTY + 3LL * kTY * (kTX + D - 1);
-        if (filt) {
-            const long long w = kTX + D + 1, rows = kTY + 4;
-            f += (long long)kTY * (kTX + 2) + (long long)kTY * w + rows * (w + 4) + rows * w;
-        }
-        return f;
+    const Geom g = geom(r, D);
+    if (kind == TDV_COST_BT) return band_floats_r<TDV_COST_BT, 0>(g, filt);
+    const bool ncc = kind == TDV_COST_NCC;
+    switch (r) {
+        case 1: return ncc ? band_floats_r<TDV_COST_NCC, 1>(g, filt) : band_floats_r<TDV_COST_SSD, 1>(g, filt);
+        case 2: return ncc ? band_floats_r<TDV_COST_NCC, 2>(g, filt) : band_floats_r<TDV_COST_SSD, 2>(g, filt);
+        case 3: return ncc ? band_floats_r<TDV_COST_NCC, 3>(g, filt) : band_floats_r<TDV_COST_SSD, 3>(g, filt);
+        default: return ncc ? band_floats_r<TDV_COST_NCC, 4>(g, filt) : band_floats_r<TDV_COST_SSD, 4>(g, filt);
     }
-    f = (long long)(kTY + 2 * r) * (lbw + rbw);
-    if (kind == TDV_COST_NCC) f += (long long)kTX * kTY + (long long)kTY * (kTX + D - 1);
-    if (filt) {
-        const long long w = lbw > rbw ? lbw : rbw, rows = kTY + 2 * r + 4;
-        f += rows * (w + 4) + rows * w;
-    }
-    return f;
 }
 
 }  // namespace
@@ -635,31 +741,28 @@ bool cost_banded_supported(int kind, int radius, int D, bool prefiltered) {
     return band_floats(kind, kind == TDV_COST_BT ? 0 : radius, D, prefiltered) * 4 <= kMaxBandBytes;
 }
 
-cudaError_t launch_fast_wta_banded(const ImgArg& L, const ImgArg& R, int D, int radius, uint16_t* disp,
-                                  float* disp_norm, cudaStream_t st) {
-    Geom g;
-    g.D = D;
-    g.Dw = D >= 32 ? 32 : D > 8 ? 16 : 8;
-    g.G = 32 / g.Dw;
-    g.lbw = left_band_width(radius);
-    g.rbw = kTX + D - 1 + 2 * radius;
+cudaError_t launch_fast_wta_banded(const ImgArg& L, const ImgArg& R, int D, int radius, bool prefiltered,
+                                  uint16_t* disp, float* disp_norm, cudaStream_t st) {
+    const Geom g = geom(radius, D);
+    if (prefiltered) {
+        switch (radius) {
+            case 1: return launch_fastwta_r<1, true>(L, R, g, disp, disp_norm, st);
+            case 2: return launch_fastwta_r<2, true>(L, R, g, disp, disp_norm, st);
+            case 3: return launch_fastwta_r<3, true>(L, R, g, disp, disp_norm, st);
+            default: return launch_fastwta_r<4, true>(L, R, g, disp, disp_norm, st);
+        }
+    }
     switch (radius) {
-        case 1: return launch_fastwta_r<1>(L, R, g, disp, disp_norm, st);
-        case 2: return launch_fastwta_r<2>(L, R, g, disp, disp_norm, st);
-        case 3: return launch_fastwta_r<3>(L, R, g, disp, disp_norm, st);
-        default: return launch_fastwta_r<4>(L, R, g, disp, disp_norm, st);
+        case 1: return launch_fastwta_r<1, false>(L, R, g, disp, disp_norm, st);
+        case 2: return launch_fastwta_r<2, false>(L, R, g, disp, disp_norm, st);
+        case 3: return launch_fastwta_r<3, false>(L, R, g, disp, disp_norm, st);
+        default: return launch_fastwta_r<4, false>(L, R, g, disp, disp_norm, st);
     }
 }
 
 cudaError_t launch_cost_banded(const ImgArg& L, const ImgArg& R, int kind, int radius, const VolArg& out,
                                bool prefiltered, float* left_filtered, cudaStream_t st) {
-    Geom g;
-    g.D = out.D;
-    g.Dw = out.D >= 32 ? 32 : out.D > 8 ? 16 : 8;
-    g.G = 32 / g.Dw;
-    const int r = kind == TDV_COST_BT ? 0 : radius;
-    g.lbw = left_band_width(r);
-    g.rbw = kTX + out.D - 1 + 2 * r;
+    const Geom g = geom(kind == TDV_COST_BT ? 0 : radius, out.D);
     if (prefiltered) {
         if (kind == TDV_COST_BT) return launch_one<TDV_COST_BT, 0, 8, true>(L, R, out, g, left_filtered, st);
         if (kind == TDV_COST_SSD) return dispatch_r<TDV_COST_SSD, true>(radius, L, R, out, g, left_filtered, st);

@@ -744,7 +744,7 @@ cudaError_t launch_dp(const VolArg& C, uint16_t* disp, float* disp_norm, void* c
 cudaError_t launch_fast_wta(const ImgArg& L, const ImgArg& R, int D, int radius, uint16_t* disp,
                             float* disp_norm, cudaStream_t st, Timer* tm) {
     if (cost_banded_supported(TDV_COST_SSD, radius, D)) {
-        const cudaError_t e = launch_fast_wta_banded(L, R, D, radius, disp, disp_norm, st);
+        const cudaError_t e = launch_fast_wta_banded(L, R, D, radius, false, disp, disp_norm, st);
         if (tm) tm->mark("fast_wta");
         return e;
     }

@@ -62,6 +62,9 @@ class StereoMatcher:
         self.cost, self.optimizer, self.median_filter = cost, optimizer, bool(median_filter)
 
     def __call__(self, left, right):
+        if self.median_filter and self.cost == "ssd" and self.optimizer == "wta" and left.shape == right.shape:
+            # filter, cost and winner in one kernel, no cost volume
+            return self.ctx.fast_wta_filtered(left, right, self.max_disp, norm=True)["disp_norm"]
         if self.median_filter:
             # the Gaussian runs inside the cost kernel; the filtered left
             # image is kept as the SGM's P2 guide

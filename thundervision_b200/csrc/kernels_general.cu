@@ -634,6 +634,152 @@ __global__ void __launch_bounds__(128) dp_kernel(VolArg C, uint8_t* codes, uint1
     }
 }
 
+// DP scanline for D a multiple of 16 up to 256 and a volume on 16 bytes (whole
+// vectors per lane): lane l holds disparities
+// NPL l .. NPL l + NPL - 1, so a step is one vector load of C, one vector store
+// of codes and one shuffle each way.  What bounds it: with one row per warp
+// (480 to 1080 warps on 592 schedulers) a scanline is one chain of W steps, so
+// the time is instructions per step: lane-interleaved disparities take two
+// loads, two stores and four shuffles per step at D = 64 (640x480: 0.119 ms,
+// here 0.087; with 8 instead of 16 columns of C in flight 0.101).
+// The backtrack's chain runs in lane 0 over codes staged in shared memory 32
+// columns at a time, the next columns' loads in flight.  Comparisons, their
+// order and the backtrack are dp_kernel's.
+template <int NPL, typename T>
+__global__ void __launch_bounds__(128) dp_run_kernel(VolArg C, uint8_t* codes, uint16_t* disp, float* disp_norm) {
+    constexpr int CW = 32;                // backtrack columns per stage
+    constexpr int SV = CW * NPL * 2;      // 16-byte vectors per stage at most
+    constexpr int SL = (SV + 31) / 32;    // ... per lane
+    __shared__ __align__(16) uint4 stage_all[4][SV];
+    __shared__ int zs_all[4][CW];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int y = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
+    if (y >= C.H) return;
+    int* const zs = zs_all[wib];
+    const int D = C.D, W = C.W;
+    const int d0 = lane * NPL;
+    const bool in = d0 < D;
+    struct alignas(NPL * sizeof(T) < 16 ? NPL * sizeof(T) : 16) Run {
+        T v[NPL];
+    };
+    struct alignas(NPL) Codes {
+        uint8_t v[NPL];
+    };
+    const T* cp = (const T*)C.ptr + y * C.sy + d0;
+    uint8_t* crow = codes + (size_t)y * W * D;
+    uint8_t* co = crow + d0;
+    auto load = [&](const T* q) {
+        Run r;
+        if (in) {
+            r = *reinterpret_cast<const Run*>(q);
+        } else {
+#pragma unroll
+            for (int j = 0; j < NPL; j++) r.v[j] = T(0);
+        }
+        return r;
+    };
+    float A[NPL];
+    {
+        const Run r = load(cp);
+        Codes one;
+#pragma unroll
+        for (int j = 0; j < NPL; j++) {
+            A[j] = in ? cdec(r.v[j]) : CUDART_INF_F;
+            one.v[j] = 1;
+        }
+        if (in) *reinterpret_cast<Codes*>(co) = one;
+    }
+    constexpr int K = NPL == 2 ? 16 : (NPL == 4 ? 8 : 4);  // columns of C in flight
+    Run ring[K];
+    cp += C.sx;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        if (1 + k < W) ring[k] = load(cp);
+        cp += C.sx;
+    }
+    for (int x0 = 1; x0 < W; x0 += K) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (x0 + k >= W) break;
+            float up = __shfl_up_sync(0xFFFFFFFFu, A[NPL - 1], 1);
+            float dn = __shfl_down_sync(0xFFFFFFFFu, A[0], 1);
+            if (lane == 0) up = CUDART_INF_F;
+            if (lane == 31) dn = CUDART_INF_F;
+            float An[NPL];
+            Codes cd;
+#pragma unroll
+            for (int j = 0; j < NPL; j++) {
+                const float c1 = j > 0 ? A[j - 1] : up, c2 = A[j], c3 = j < NPL - 1 ? A[j + 1] : dn;
+                float m;
+                if (c1 < c2 && c1 < c3) { m = c1; cd.v[j] = 0; }
+                else if (c2 < c3) { m = c2; cd.v[j] = 1; }
+                else { m = c3; cd.v[j] = 2; }
+                An[j] = in ? __fadd_rn(cdec(ring[k].v[j]), m) : CUDART_INF_F;
+            }
+            co += D;
+            if (in) *reinterpret_cast<Codes*>(co) = cd;
+#pragma unroll
+            for (int j = 0; j < NPL; j++) A[j] = An[j];
+            if (x0 + k + K < W) ring[k] = load(cp);
+            cp += C.sx;
+        }
+    }
+    // argmin of the last column, strict '<' from d = 0; a NaN at d = 0 pins it
+    uint32_t bo = 0xFFFFFFFFu;
+    int bd = 0x7FFFFFFF;
+#pragma unroll
+    for (int j = 0; j < NPL; j++)
+        if (in) argmin_merge(bo, bd, ford(A[j]), d0 + j);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t o2 = __shfl_xor_sync(0xFFFFFFFFu, bo, s);
+        const int d2 = __shfl_xor_sync(0xFFFFFFFFu, bd, s);
+        argmin_merge(bo, bd, o2, d2);
+    }
+    const bool nan0 = __shfl_sync(0xFFFFFFFFu, A[0] != A[0] ? 1 : 0, 0) != 0;
+    int z = (bd == 0x7FFFFFFF || nan0) ? 0 : bd;
+    // the codes written above must be visible to the warp's staging loads
+    __syncwarp();
+    __threadfence_block();
+    // columns [xs, xe] of this row's codes, as 16-byte vectors
+    const uint8_t* const stage = reinterpret_cast<const uint8_t*>(stage_all[wib]);
+    uint4 pre[SL];
+    auto fetch = [&](int xe) {
+        const int xs = max(0, xe - CW + 1);
+        const uint4* src = reinterpret_cast<const uint4*>(crow + (size_t)xs * D);
+        const int n = ((xe - xs + 1) * D + 15) >> 4;
+#pragma unroll
+        for (int i = 0; i < SL; i++)
+            if (lane + 32 * i < n) pre[i] = src[lane + 32 * i];
+    };
+    fetch(W - 1);
+    for (int xe = W - 1; xe >= 0; xe -= CW) {
+        const int xs = max(0, xe - CW + 1);
+        const int n = ((xe - xs + 1) * D + 15) >> 4;
+#pragma unroll
+        for (int i = 0; i < SL; i++)
+            if (lane + 32 * i < n) stage_all[wib][lane + 32 * i] = pre[i];
+        __syncwarp();
+        if (xe - CW >= 0) fetch(xe - CW);
+        if (lane == 0) {
+            for (int x = xe; x >= xs; x--) {
+                const int nz = z + (int)stage[(x - xs) * D + z] - 1;
+                if (nz >= 0 && nz < D) z = nz;
+                zs[x - xs] = z;
+            }
+        }
+        __syncwarp();
+        z = __shfl_sync(0xFFFFFFFFu, z, 0);
+        if (lane <= xe - xs) {
+            const size_t o = (size_t)y * W + xs + lane;
+            const int zz = zs[lane];
+            if (disp) disp[o] = (uint16_t)zz;
+            if (disp_norm) disp_norm[o] = __fdiv_rn((float)zz, (float)D);
+        }
+        __syncwarp();
+    }
+}
+
 // SSD window + argmin fused (tdvision/fastwta.cu:32-53), one thread per pixel.
 __global__ void fast_wta_kernel(ImgArg L, ImgArg R, int D, int r, uint16_t* disp, float* disp_norm) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -722,6 +868,21 @@ cudaError_t launch_dp(const VolArg& C, uint16_t* disp, float* disp_norm, void* c
     const int blocks = (C.H + 3) / 4;
     const int D = C.D;
     uint8_t* cd = (uint8_t*)codes;
+    // whole vectors per lane: 16-byte multiples of codes per column too, so
+    // that the backtrack's stages start aligned
+    if (D % 16 == 0 && D <= 256 && (((uintptr_t)C.ptr | (uintptr_t)codes) & 15) == 0) {
+        if (C.u16) {
+            if (D <= 64) dp_run_kernel<2, uint16_t><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+            else if (D <= 128) dp_run_kernel<4, uint16_t><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+            else dp_run_kernel<8, uint16_t><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+        } else {
+            if (D <= 64) dp_run_kernel<2, float><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+            else if (D <= 128) dp_run_kernel<4, float><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+            else dp_run_kernel<8, float><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
+        }
+        if (tm) tm->mark("dp_scanline");
+        return cudaGetLastError();
+    }
     if (C.u16) {
         if (D <= 32) dp_kernel<1, uint16_t><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);
         else if (D <= 64) dp_kernel<2, uint16_t><<<blocks, 128, 0, st>>>(C, cd, disp, disp_norm);

@@ -74,17 +74,45 @@ def test_two_lines_per_lane_group(ctx, orc, sem, table):
     _check(ctx, orc, 1205, 61, 136, sem=sem, table=table, seed=2)
 
 
-@pytest.mark.parametrize("W,H,D", [(640, 480, 64), (501, 333, 100), (1280, 353, 256)])
-def test_equals_accumulating_passes(ctx, W, H, D):
-    """The same pair through a batch, which runs the accumulating passes."""
-    left, right, _, _ = syn.make_pair(W, H, D, 3, n_rects=8, slanted=True, salt_pepper=0.02)
-    lt, rt = torch.from_numpy(left).cuda(), torch.from_numpy(right).cuda()
-    a = ctx.stereo_sgm(lt, rt, D, 10, 120, lr=1, right_disp=True)
-    b = api.Batch(ctx, [(lt, rt, D)], 10, 120, lr=1, right_disp=True)
-    r = b.run()[0]
-    b.status()
-    for k in ("disp", "disp_right"):
-        assert torch.equal(a[k].to(torch.int32), r[k].to(torch.int32))
+@pytest.mark.parametrize("p2,paths", [(120, 8), (120, 4), (128, 8), (300.5, 4)])
+def test_batch_on_both_sides_of_the_range_rule(ctx, p2, paths):
+    """Batches store the directions apart up to P2 = 127.5 and accumulate above;
+    both equal the per-pair calls."""
+    pairs = []
+    for i, (W, H, D, lr) in enumerate([(70, 40, 12, 1), (333, 61, 32, None), (96, 130, 64, 2), (240, 33, 100, None),
+                                       (501, 29, 200, 1), (5, 3, 8, 1)]):
+        left, right, _, _ = syn.make_pair(max(W, 40), max(H, 30), D, 40 + i, n_rects=3)
+        cut = lambda a: torch.from_numpy(np.ascontiguousarray(a[:H, :W])).cuda()
+        pairs.append((cut(left), cut(right), D, lr))
+    b = api.Batch(ctx, pairs, 10, p2, paths=paths, norm=True, right_disp="lr")
+    for _ in range(2):
+        out = b.run()
+        b.status()
+        for (lt, rt, D, lr), o in zip(pairs, out):
+            want = ctx.stereo_sgm(lt, rt, D, 10, p2, paths=paths, lr=lr, norm=True, right_disp=lr is not None)
+            for k in want:
+                assert torch.equal(o[k].view(torch.int32 if k == "disp_norm" else torch.int16),
+                                   want[k].view(torch.int32 if k == "disp_norm" else torch.int16))
+    b.close()
+
+
+@pytest.mark.slow
+def test_batch_waves(ctx):
+    """Three full-HD pairs at D = 256 and a small one: more volumes than one wave holds."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    pairs = []
+    for W, H, D in [(1920, 1080, 256), (1920, 1080, 256), (64, 48, 32), (1920, 1080, 200)]:
+        left = torch.randint(0, 256, (H, W), generator=g, device="cuda", dtype=torch.uint8)
+        pairs.append((left, torch.roll(left, -9, 1), D, 1))
+    b = api.Batch(ctx, pairs, 10, 120)
+    for order in (0, 1):
+        b.set_tiles(order=order)
+        out = b.run()
+        b.status()
+        for (lt, rt, D, lr), o in zip(pairs, out):
+            want = ctx.stereo_sgm(lt, rt, D, 10, 120, lr=lr)["disp"]
+            assert torch.equal(o["disp"].view(torch.int16), want.view(torch.int16))
     b.close()
 
 

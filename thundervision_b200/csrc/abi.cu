@@ -1077,6 +1077,7 @@ struct tdv_batch {
     tdv_batch_tiles tiles{};
     tdv::BatchPlan plan;
     void* scratch = nullptr;
+    bool dirs = false;  // every direction stored apart (kernels_dirs.cu)
     void* desc = nullptr;
     size_t desc_bytes = 0;
     cudaGraphExec_t gexec = nullptr;
@@ -1114,7 +1115,7 @@ tdv_status batch_replan(tdv_batch* b, const tdv_batch_tiles& t) {
     tdv_ctx* ctx = b->ctx;
     for (int pass = 0; pass < 2; pass++) {
         tdv::BatchPlan plan;
-        const char* msg = tdv::batch_plan(b->pairs, b->p1h, b->p2h, b->paths, t, (unsigned char*)b->scratch,
+        const char* msg = tdv::batch_plan(b->pairs, b->p1h, b->p2h, b->paths, t, b->dirs, (unsigned char*)b->scratch,
                                           (unsigned char*)b->desc, plan);
         if (msg) return fail(ctx, TDV_ERR_UNSUPPORTED, "batch tiles: %s", msg);
         if (plan.bytes > b->desc_bytes) {
@@ -1198,8 +1199,12 @@ tdv_status tdv_batch_create(tdv_ctx* ctx, const tdv_batch_pair* pairs, int32_t n
         delete b;
         return fail(ctx, TDV_ERR_CUDA, "querying the SM count failed");
     }
+    // every direction stored apart where the range and the memory allow
+    const size_t db = tdv::batch_dirs_scratch_bytes(b->pairs, b->p1h, b->p2h, b->paths);
+    if (db) b->scratch = dev_alloc(ctx, db);
+    b->dirs = b->scratch != nullptr;
     const size_t sb = tdv::batch_scratch_bytes(b->pairs);
-    b->scratch = dev_alloc(ctx, sb);
+    if (!b->dirs) b->scratch = dev_alloc(ctx, sb);
     if (!b->scratch) {
         delete b;
         return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of batch scratch failed", sb);

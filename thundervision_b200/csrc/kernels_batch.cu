@@ -224,11 +224,16 @@ size_t batch_scratch_bytes(const std::vector<BatchPairArgs>& pairs) {
 }
 
 const char* batch_plan(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths,
-                       const BatchTiles& t, unsigned char* scratch, unsigned char* d_desc, BatchPlan& out) {
+                       const BatchTiles& t, bool dirs, unsigned char* scratch, unsigned char* d_desc, BatchPlan& out) {
     const int n = (int)pairs.size();
     if (t.lines_per_cta < 1 || t.lines_per_cta > kMaxG) return "lines_per_cta must be in [1, 24]";
     if (t.rows_per_cta < 1 || t.rows_per_cta > kBatchWarps) return "rows_per_cta must be in [1, 25]";
     if (t.ctas_per_sm != 1 && t.ctas_per_sm != 2) return "ctas_per_sm must be 1 or 2";
+    if (dirs) {
+        // its tiles follow from each pair's lanes per line; the queue order stays the caller's
+        batch_dirs_plan(pairs, p1h, p2h, paths, t.order == TDV_BATCH_ORDER_LONGEST_FIRST, scratch, d_desc, out);
+        return nullptr;
+    }
     const int NW = t.ctas_per_sm == 2 ? kBatchWarps2 : kBatchWarps;
     const int budget = t.ctas_per_sm == 2 ? kSmemBudget2 : kSmemBudget;
     std::vector<BPair> hp(n);
@@ -371,11 +376,13 @@ cudaError_t configure_nw(const BatchPlan& plan) {
 }
 
 cudaError_t batch_configure(const BatchPlan& plan) {
+    if (plan.dirs) return batch_dirs_configure(plan);
     return plan.ctas_per_sm == 2 ? configure_nw<kBatchWarps2>(plan) : configure_nw<kBatchWarps>(plan);
 }
 
 cudaError_t batch_launch(const BatchPlan& plan, unsigned char* d_desc, unsigned long long wait_ns, int grid,
                          cudaStream_t st, unsigned long long* trace) {
+    if (plan.dirs) return batch_dirs_launch(plan, d_desc, wait_ns, grid, st, trace);
     cudaError_t e = cudaMemsetAsync(d_desc + plan.ctl_off, 0, batch_ctl_bytes(plan.n_pairs), st);
     if (e != cudaSuccess) return e;
     const BPair* pairs = (const BPair*)(d_desc + plan.pairs_off);

@@ -48,6 +48,8 @@
 // Which directions count in a pixel, and how often, is applied by the sum.
 #include <algorithm>
 #include <atomic>
+#include <cstring>
+#include <vector>
 
 #include "fused_body.cuh"
 
@@ -69,11 +71,12 @@ constexpr uint32_t kCorner = 0x100u;      // pixel flag: some direction counts m
 // all but one of their right-plane entries (5 loads instead of 8, and two
 // independent recurrences in flight), which pays where a line fills half a
 // warp or more; with shorter lines the warp already walks 4 to 16.
-template <int LPG, int LN_>
+// NWB: consumer warps where the caller's block fixes them (0: the launch's own).
+template <int LPG, int LN_, int NWB = 0>
 struct Cfg {
     static constexpr int NSUB = 32 / LPG;
     static constexpr int LN = LN_;
-    static constexpr int NW = LPG == 32 ? 8 : (LPG == 16 ? 4 : 3);
+    static constexpr int NW = NWB ? NWB : (LPG == 32 ? 8 : (LPG == 16 ? 4 : 3));
     static constexpr int G = NW * NSUB * LN;          // lines per vertical / diagonal block
     static constexpr int RH = NW * NSUB;              // rows per horizontal block
     static constexpr int T = (NW + 1) * 32;
@@ -243,13 +246,19 @@ __device__ __forceinline__ uint3 bt_plane(const ImgArg& im, int x, int y) {
     return make_uint3(2 * i2, mx + mn, mx - mn);
 }
 
+__device__ __forceinline__ void dirs_prep_pixel(const ImgArg& L, const ImgArg& R, uint4* LP, uint4* RP, int W, int x,
+                                                int y, uint32_t dirs) {
+    const uint3 l = bt_plane(L, x, y);
+    LP[(size_t)y * W + x] = make_uint4(l.x * 0x10001u, l.y * 0x10001u, l.z * 0x10001u, dirs);
+    const uint3 a = bt_plane(R, x, y), b = bt_plane(R, max(x - 4, 0), y);
+    RP[(size_t)y * W + x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), 0);
+}
+
 __global__ void dirs_prep_kernel(ImgArg L, ImgArg R, uint4* LP, uint4* RP, int W, int H, int nd,
                                  const uint8_t* lw, const uint8_t* bw, const int* corner, int nl, int nb) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;
-    const uint3 l = bt_plane(L, x, y);
-    const uint32_t active = nd == 8 ? 0xFFu : 0x0Fu;
-    uint32_t dirs = active;
+    uint32_t dirs = nd == 8 ? 0xFFu : 0x0Fu;
     if (lw) {
         const bool border = y == 0 || y == H - 1 || x == 0 || x == W - 1;
         dirs = 0;
@@ -262,9 +271,7 @@ __global__ void dirs_prep_kernel(ImgArg L, ImgArg R, uint4* LP, uint4* RP, int W
         }
         if (corner && (corner[4 * y] == x || corner[4 * y + 2] == x)) dirs |= kCorner;
     }
-    LP[(size_t)y * W + x] = make_uint4(l.x * 0x10001u, l.y * 0x10001u, l.z * 0x10001u, dirs);
-    const uint3 a = bt_plane(R, x, y), b = bt_plane(R, max(x - 4, 0), y);
-    RP[(size_t)y * W + x] = make_uint4(a.x | (b.x << 16), a.y | (b.y << 16), a.z | (b.z << 16), 0);
+    dirs_prep_pixel(L, R, LP, RP, W, x, y, dirs);
 }
 
 // ---------------------------------------------- vertical / diagonal lines
@@ -287,10 +294,10 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
 // and cost a diagonal step 14 instructions of addressing more); one 16-byte
 // slot after every 8 entries keeps lanes reading entries 8 apart on distinct
 // banks.
-template <int LPG, int LNT, int EXCL>
+template <int LPG, int LNT, int EXCL, int NWB = 0>
 __device__ __forceinline__ void lines_vd(const EK& k, int dir, int s, int dy, int grp, const uint4* masks,
                                          unsigned char* smem) {
-    using C = Cfg<LPG, LNT>;
+    using C = Cfg<LPG, LNT, NWB>;
     constexpr int LN = C::LN, G = C::G, DS = C::DS, U = kRowsPerSlot, NS = kSlots, NR = 3 + LN;
     constexpr int offR = G * 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -496,7 +503,7 @@ struct Window {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int e = min(max(x0 - j, 0), width - 1), f = min(max(x0 - j - 4, 0), width - 1);
-            const uint4 a = __ldg(rrow + e), b = __ldg(rrow + f);
+            const uint4 a = __ldca(rrow + e), b = __ldca(rrow + f);
             I[j] = __byte_perm(a.x, b.x, 0x5410);
             S[j] = __byte_perm(a.y, b.y, 0x5410);
             W[j] = __byte_perm(a.z, b.z, 0x5410);
@@ -545,9 +552,9 @@ struct Window {
 // pair j holding o = j (low) and o = j + 4 (high); per step one value enters
 // the lane from its neighbour (one shuffle and one permute per plane) and the
 // pairs rotate by one register.
-template <int LPG, int LNT, int EXCL, bool DXP>
+template <int LPG, int LNT, int EXCL, bool DXP, int NWB = 0>
 __device__ __forceinline__ void lines_h(const EK& k, int dir, int grp, const uint4* masks, unsigned char* smem) {
-    using C = Cfg<LPG, LNT>;
+    using C = Cfg<LPG, LNT, NWB>;
     constexpr int CH = C::CH, KC = C::KC, DS = C::DS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / LPG, sl = lane & (LPG - 1);
@@ -577,8 +584,8 @@ __device__ __forceinline__ void lines_h(const EK& k, int dir, int grp, const uin
         for (int i = 0; i < KC; i++) {
             const int t = t0 + sl + i * LPG;
             const int x = xpos(min(t, W - 1)), e = epos(t);
-            nl[i] = __ldg(lrow + x);
-            nr[i] = __ldg(rrow + e);
+            nl[i] = __ldca(lrow + x);
+            nr[i] = __ldca(rrow + e);
         }
     };
     uint32_t L[1][4] = {{0, 0, 0, 0}}, MM[1] = {0};
@@ -649,18 +656,14 @@ __device__ __forceinline__ void lines_h(const EK& k, int dir, int grp, const uin
     }
 }
 
-// Every line of every direction.  Blocks are handed out in index order, the
-// long ones first: the horizontal lines (W steps; after the vertical ones in
+// One block's lines.  Blocks are handed out in index order,
+// the long ones first: the horizontal lines (W steps; after the vertical ones in
 // portrait images), the vertical, then the diagonal groups from the middle of
-// their range outwards (their lengths fall towards the image corners).
-template <int LPG, int LNT, int EXCL>
-__global__ void __launch_bounds__(Cfg<LPG, LNT>::T, Cfg<LPG, LNT>::MINB) dirs_pass_kernel(EK k, int nh, int nv, int ng) {
-    extern __shared__ __align__(128) unsigned char smem_all[];
-    const uint4* masks = (const uint4*)smem_all;
-    unsigned char* smem = smem_all + kMaskBytes;
-    mask_table((uint4*)smem_all, k.BIG2);
-    __syncthreads();
-    int b = blockIdx.x;
+// their range outwards (their lengths fall towards the image corners).  Returns
+// whether the block set up barriers.
+template <int LPG, int LNT, int EXCL, int NWB = 0>
+__device__ __forceinline__ bool lines_block(const EK& k, int b, int nh, int nv, int ng, const uint4* masks,
+                                            unsigned char* smem) {
     int kind;  // 0 horizontal, 1 vertical, 2 diagonal
     if (k.W >= k.H) {
         kind = b < nh ? 0 : (b < nh + nv ? 1 : 2);
@@ -670,21 +673,33 @@ __global__ void __launch_bounds__(Cfg<LPG, LNT>::T, Cfg<LPG, LNT>::MINB) dirs_pa
         b -= kind == 1 ? 0 : (kind == 0 ? nv : nh + nv);
     }
     if (kind == 0) {
-        if ((b & 1) == 0) lines_h<LPG, LNT, EXCL, true>(k, 2, b >> 1, masks, smem);
-        else lines_h<LPG, LNT, EXCL, false>(k, 3, b >> 1, masks, smem);
-        return;
+        if ((b & 1) == 0) lines_h<LPG, LNT, EXCL, true, NWB>(k, 2, b >> 1, masks, smem);
+        else lines_h<LPG, LNT, EXCL, false, NWB>(k, 3, b >> 1, masks, smem);
+        return false;
     }
     int dir = b & 1, s = 0, dy = (b & 1) ? -1 : 1, g = b >> 1;
     if (kind == 2) {
         const int d = b & 3, i = b >> 2;
         const int mid = ng >> 1;
         g = (i & 1) ? mid - ((i + 1) >> 1) : mid + (i >> 1);  // mid, mid-1, mid+1, ...
-        if (g < 0 || g >= ng) return;
+        if (g < 0 || g >= ng) return false;
         // D1+ (1,1) D1- (-1,-1) D2+ (-1,1) D2- (1,-1)
         dir = 4 + d;
         s = d < 2 ? 1 : -1;
     }
-    lines_vd<LPG, LNT, EXCL>(k, dir, s, dy, g, masks, smem);
+    lines_vd<LPG, LNT, EXCL, NWB>(k, dir, s, dy, g, masks, smem);
+    return true;
+}
+
+// Every line of every direction.
+template <int LPG, int LNT, int EXCL>
+__global__ void __launch_bounds__(Cfg<LPG, LNT>::T, Cfg<LPG, LNT>::MINB) dirs_pass_kernel(EK k, int nh, int nv, int ng) {
+    extern __shared__ __align__(128) unsigned char smem_all[];
+    const uint4* masks = (const uint4*)smem_all;
+    unsigned char* smem = smem_all + kMaskBytes;
+    mask_table((uint4*)smem_all, k.BIG2);
+    __syncthreads();
+    lines_block<LPG, LNT, EXCL>(k, blockIdx.x, nh, nv, ng, masks, smem);
 }
 
 // ------------------------------------------------------------------- sum
@@ -709,13 +724,13 @@ constexpr int kSumMaxThreads = 512;  // at most 128 registers a thread: 16 warps
 // D = 256 it reads 4.25 GB once; each warp keeps the bytes of two pixels in
 // flight.
 template <int LPG, int ND, bool WTD, bool EXCL, bool LR>
-__global__ void __launch_bounds__(kSumMaxThreads, 1) dirs_sum_kernel(EK k, SumOut o) {
-    extern __shared__ __align__(16) int rowR_all[];  // [rows][W] keys, then [rows][W] u16 left disparities
+__device__ __forceinline__ void sum_rows(const EK& k, const SumOut& o, int blk, int* rowR_all) {
+    // rowR_all: [rows][W] keys (LR), then [rows][W] u16 left disparities
     constexpr int NSUB = 32 / LPG, DS = 8 * LPG;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / LPG, sl = lane & (LPG - 1);
     const int W = k.W;
-    const int yb = blockIdx.x * o.rows;
+    const int yb = blk * o.rows;
     const int nrows = min(o.rows, k.H - yb);
     uint16_t* rowL_all = (uint16_t*)(rowR_all + (LR ? o.rows * W : 0));
     if (LR) {
@@ -768,8 +783,8 @@ __global__ void __launch_bounds__(kSumMaxThreads, 1) dirs_sum_kernel(EK k, SumOu
                     x2[B][d + 3] = v.w;
                 }
             }
-            lp2[B] = __ldg(lrow + xx);
-            if (loader) ed2[B] = __ldg(rrow + max(x - DS + 1, 0));
+            lp2[B] = __ldca(lrow + xx);
+            if (loader) ed2[B] = __ldca(rrow + max(x - DS + 1, 0));
         };
         auto step = [&](auto Tc, int x) {
             constexpr int T = decltype(Tc)::value;
@@ -923,6 +938,167 @@ __global__ void __launch_bounds__(kSumMaxThreads, 1) dirs_sum_kernel(EK k, SumOu
     }
 }
 
+template <int LPG, int ND, bool WTD, bool EXCL, bool LR>
+__global__ void __launch_bounds__(kSumMaxThreads, 1) dirs_sum_kernel(EK k, SumOut o) {
+    extern __shared__ __align__(16) int sum_smem[];
+    sum_rows<LPG, ND, WTD, EXCL, LR>(k, o, blockIdx.x, sum_smem);
+}
+
+// ------------------------------------------------------------------ batch
+// The pairs of a batch (kernels_batch.cu: a work queue taken by persistent
+// blocks) in three steps: prep, the lines of every direction, the sum.  The
+// queue is pass-major, so pairs' lines fill the chip together, and a pair's
+// only waits are for its own prep and lines: with passes accumulating into one
+// S a pair is a chain of nine.  Lines and sums are launches of their own (three
+// blocks of 8 consumer warps and a producer per SM at 72 registers; two blocks
+// of 8 warps at 128): in one kernel the sums' registers leave 16 warps per SM
+// to the lines, or spill (16 pairs, 2.0 G cells: 15.7 ms in one, 10.8 in two,
+// 16.8 with accumulating passes).  The pairs go in waves whose volumes share
+// one region of kWaveBytes (at most kWaves waves), so a large batch needs no
+// more memory than its accumulation volumes would: pass 0 is every pair's prep,
+// 1 + 2w the lines and 2 + 2w the sums of wave w.
+constexpr int kBatchNW = 8;
+constexpr int kBatchT = (kBatchNW + 1) * 32;
+constexpr int kBatchSumT = kBatchNW * 32;
+constexpr int kSteps = 3;
+constexpr int kWaves = 7;
+constexpr size_t kWaveBytes = (size_t)8 << 30;
+constexpr int kDirsPrepPixels = 8192;  // pixels per prep item
+constexpr int kDirsCtlHeader = 16;     // ints: spare, error word, the launches' queue heads
+
+struct DPair {
+    EK k;
+    ImgArg L, R;
+    SumOut o;
+    int lpg, nh, nv, ng, prep_rows, lr, wave;
+    int nb[kSteps];
+};
+struct DItem {
+    int32_t pp;   // pair * 16 + pass
+    int32_t blk;  // block index inside the pass
+};
+
+__device__ __forceinline__ int acquire_load(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+// Waits until *cnt >= target; false on timeout (recorded) or on an error
+// recorded by another block.
+__device__ bool wait_count(const int* cnt, int target, int* err, uint64_t limit_ns) {
+    if (acquire_load(cnt) >= target) return true;
+    const uint64_t t0 = global_ns();
+    for (;;) {
+        __nanosleep(200);
+        if (acquire_load(cnt) >= target) return true;
+        if (*(volatile int*)err != 0) return false;
+        if (global_ns() - t0 > limit_ns) {
+            atomicCAS(err, 0, (int)TDV_ERR_TIMEOUT);
+            return false;
+        }
+    }
+}
+
+template <int LPG, int LNT, int ND, bool SUM>
+__device__ __forceinline__ bool batch_item(const DPair& sp, int blk, const uint4* masks, unsigned char* smem) {
+    const EK k = sp.k;
+    if constexpr (!SUM) {
+        return lines_block<LPG, LNT, 0, kBatchNW>(k, blk, sp.nh, sp.nv, sp.ng, masks, smem);
+    } else {
+        const SumOut o = sp.o;
+        if (sp.lr) sum_rows<LPG, ND, false, false, true>(k, o, blk, (int*)smem);
+        else sum_rows<LPG, ND, false, false, false>(k, o, blk, (int*)smem);
+        return false;
+    }
+}
+
+// Items first .. last-1 of the queue: (prep and) lines, or (SUM) sums.
+template <int ND, bool SUM>
+__global__ void __launch_bounds__(SUM ? kBatchSumT : kBatchT, SUM ? 2 : 3)
+    batch_dirs_kernel(const DPair* __restrict__ pairs, int npairs, const DItem* __restrict__ items, int first, int last, int head_at, int* ctl,
+                      unsigned long long wait_ns, unsigned long long* trace) {
+    extern __shared__ __align__(128) unsigned char smem_all[];
+    __shared__ DPair sp;
+    __shared__ int s_pass, s_blk, s_stop, s_slot, s_item, s_pp;
+    __shared__ unsigned long long s_take, s_go;
+    int* head = ctl + head_at;
+    int* err = ctl + 1;
+    int* done = ctl + kDirsCtlHeader;
+    const uint4* masks = (const uint4*)smem_all;
+    unsigned char* smem = smem_all + kMaskBytes;
+    if (!SUM) mask_table((uint4*)smem_all, pairs[0].k.BIG2);  // the same for every pair
+
+    for (;;) {
+        if (threadIdx.x == 0) {
+            int stop = 1;
+            if (*(volatile int*)err == 0) {
+                const int i = first + atomicAdd(head, 1);
+                s_item = i;
+                if (trace) s_take = global_ns();
+                if (i < last) {
+                    const DItem it = items[i];
+                    s_pp = it.pp;
+                    const unsigned pair = (unsigned)it.pp >> 4;
+                    const int pass = it.pp & 15;
+                    const int step = pass == 0 ? 0 : 1 + ((pass - 1) & 1);
+                    if (pair >= (unsigned)npairs || (step == 2) != SUM ||
+                        (step > 0 && pairs[pair].wave != (pass - 1) >> 1) || it.blk < 0 ||
+                        it.blk >= pairs[pair].nb[step]) {
+                        atomicCAS(err, 0, (int)TDV_ERR_BAD_WORK);
+                    } else if (step == 0 || wait_count(done + pair * kSteps + step - 1, pairs[pair].nb[step - 1], err,
+                                                       wait_ns)) {
+                        stop = 0;
+                        sp = pairs[pair];
+                        s_pass = pass;
+                        s_blk = it.blk;
+                        s_slot = pair * kSteps + step;
+                        if (trace) s_go = global_ns();
+                    }
+                }
+            }
+            s_stop = stop;
+        }
+        __syncthreads();
+        if (s_stop) break;
+        const int pass = s_pass, blk = s_blk;
+        bool barriers = false;
+        if (!SUM && pass == 0) {
+            const int W = sp.k.W, y0 = blk * sp.prep_rows, y1 = min(sp.k.H, y0 + sp.prep_rows);
+            const int n = (y1 - y0) * W;
+            for (int i = threadIdx.x; i < n; i += blockDim.x)
+                dirs_prep_pixel(sp.L, sp.R, const_cast<uint4*>(sp.k.LP), const_cast<uint4*>(sp.k.RP), W, i % W,
+                                y0 + i / W, 0xFFu);
+        } else {
+            switch (sp.lpg) {
+                case 2: barriers = batch_item<2, 1, ND, SUM>(sp, blk, masks, smem); break;
+                case 4: barriers = batch_item<4, 1, ND, SUM>(sp, blk, masks, smem); break;
+                case 8: barriers = batch_item<8, 1, ND, SUM>(sp, blk, masks, smem); break;
+                case 16: barriers = batch_item<16, 1, ND, SUM>(sp, blk, masks, smem); break;
+                default: barriers = batch_item<32, 2, ND, SUM>(sp, blk, masks, smem); break;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            // the ring's barriers are set up again by the next item that uses them
+            if (barriers)
+                for (int b = 0; b < 2 * kSlots; b++) mbar_inval(smem_u32((uint64_t*)smem + b));
+            __threadfence();
+            atomicAdd(done + s_slot, 1);
+            if (trace) {
+                unsigned smid;
+                asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+                unsigned long long* t = trace + 4 * (size_t)s_item;
+                t[0] = s_take;
+                t[1] = s_go;
+                t[2] = global_ns();
+                t[3] = ((unsigned long long)smid << 32) | (unsigned)s_pp;
+            }
+        }
+        // s_stop and the queue words are written again by thread 0 only, which
+        // every other thread waits for at the loop's barrier
+    }
+}
+
 // ------------------------------------------------------------- host side
 int lanes_for(int D) { return D <= 16 ? 2 : (D <= 32 ? 4 : (D <= 64 ? 8 : (D <= 128 ? 16 : 32))); }
 
@@ -933,14 +1109,21 @@ uint32_t enc16(uint32_t v) {
     return 3072 + (v - 4096) / 4;
 }
 
+// Blocks of the horizontal, vertical and diagonal lines (ng groups per
+// diagonal direction; the order mid, mid-1, mid+1, ... takes ng + 1 indices).
+template <typename C>
+int line_blocks(int W, int H, int paths, int& nh, int& nv, int& ng) {
+    nh = 2 * ((H + C::RH - 1) / C::RH);
+    nv = 2 * ((W + C::G - 1) / C::G);
+    ng = paths == 8 ? (W + H - 1 + C::G - 1) / C::G : 0;
+    return nh + nv + 4 * (ng ? ng + 1 : 0);
+}
+
 template <int LPG, int LNT, int EXCL>
 cudaError_t launch_dirs_pass(const EK& k, cudaStream_t st) {
     using C = Cfg<LPG, LNT>;
-    const int nh = 2 * ((k.H + C::RH - 1) / C::RH);
-    const int nv = 2 * ((k.W + C::G - 1) / C::G);
-    const int ng = k.nd == 8 ? (k.W + k.H - 1 + C::G - 1) / C::G : 0;
-    // the diagonal order mid, mid-1, mid+1, ... visits ng + 1 indices for even ng
-    const int nd = 4 * (ng ? ng + 1 : 0);
+    int nh, nv, ng;
+    const int blocks = line_blocks<C>(k.W, k.H, k.nd, nh, nv, ng);
     static std::atomic<unsigned long long> opted{0};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -950,7 +1133,7 @@ cudaError_t launch_dirs_pass(const EK& k, cudaStream_t st) {
         if (e != cudaSuccess) return e;
         if (dev < 64) opted.fetch_or(1ull << dev);
     }
-    dirs_pass_kernel<LPG, LNT, EXCL><<<nh + nv + nd, C::T, C::SMEM, st>>>(k, nh, nv, ng);
+    dirs_pass_kernel<LPG, LNT, EXCL><<<blocks, C::T, C::SMEM, st>>>(k, nh, nv, ng);
     return cudaGetLastError();
 }
 
@@ -1093,6 +1276,204 @@ cudaError_t launch_dirs(const FusedArgs& a, cudaStream_t st, Timer* tm) {
         case 16: return run_dirs<16>(k, o, wtd, a.excl != 0, lr, st, tm);
         default: return run_dirs<32>(k, o, wtd, a.excl != 0, lr, st, tm);
     }
+}
+
+// ----------------------------------------------------------- batch, host side
+namespace {
+
+template <int LPG, int LN>
+void fill_lines(DPair& P) {
+    using C = Cfg<LPG, LN, kBatchNW>;
+    P.nb[1] = line_blocks<C>(P.k.W, P.k.H, P.k.nd, P.nh, P.nv, P.ng);
+}
+
+int dirs_batch_smem(int lpg) {
+    switch (lpg) {
+        case 2: return Cfg<2, 1, kBatchNW>::SMEM;
+        case 4: return Cfg<4, 1, kBatchNW>::SMEM;
+        case 8: return Cfg<8, 1, kBatchNW>::SMEM;
+        case 16: return Cfg<16, 1, kBatchNW>::SMEM;
+        default: return Cfg<32, 2, kBatchNW>::SMEM;
+    }
+}
+
+size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// The volumes' region: kWaveBytes, or less when the batch's all fit, or what
+// kWaves greedy waves need.
+size_t wave_bytes(const std::vector<BatchPairArgs>& pairs, int paths) {
+    size_t total = 0, most = 0;
+    for (const auto& p : pairs) {
+        const size_t v = up256(dirs_bytes(p.W, p.H, p.D, paths, 0));
+        total += v;
+        most = std::max(most, v);
+    }
+    return std::min(total, std::max(kWaveBytes, total / kWaves + most));
+}
+
+}  // namespace
+
+size_t batch_dirs_scratch_bytes(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths) {
+    size_t b = 0;
+    for (const auto& p : pairs) {
+        if (!dirs_supported(p.W, p.H, p.D, p1h, p2h, 0) || (size_t)p.W * 6 > 100 * 1024) return 0;
+        b += up256(dirs_plane_bytes(p.W, p.H));
+    }
+    return b + wave_bytes(pairs, paths);
+}
+
+void batch_dirs_plan(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths, bool longest_first,
+                     unsigned char* scratch, unsigned char* d_desc, BatchPlan& out) {
+    const int n = (int)pairs.size();
+    std::vector<DPair> hp(n);
+    out.ctl_off = 0;
+    // queue order, waves and the volumes' places
+    std::vector<int> idx(n);
+    for (int i = 0; i < n; i++) idx[i] = i;
+    if (longest_first)
+        std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) {
+            return (double)pairs[x].W * lanes_for(pairs[x].D) > (double)pairs[y].W * lanes_for(pairs[y].D);
+        });
+    size_t planes = 0;
+    for (const auto& p : pairs) planes += up256(dirs_plane_bytes(p.W, p.H));
+    const size_t region = wave_bytes(pairs, paths);
+    std::vector<size_t> vol_at(n);
+    int waves = 0;
+    size_t used = 0;
+    for (int i : idx) {
+        const size_t v = up256(dirs_bytes(pairs[i].W, pairs[i].H, pairs[i].D, paths, 0));
+        if (used + v > region) {
+            waves++;
+            used = 0;
+        }
+        hp[i].wave = waves;
+        vol_at[i] = planes + used;
+        used += v;
+    }
+    out.waves = waves + 1;
+    size_t off = 0;
+    int smem = 0, sum_smem = 0;
+    const uint32_t big = (511 + 2 * (uint32_t)p2h + 11) & ~3u;
+    for (int i = 0; i < n; i++) {
+        const BatchPairArgs& a = pairs[i];
+        DPair& P = hp[i];
+        const int wave = P.wave;
+        P = DPair{};
+        P.wave = wave;
+        EK& k = P.k;
+        uint4* LP = (uint4*)(scratch + off) + kGuard;
+        k.LP = LP;
+        k.RP = LP + (size_t)a.W * a.H + 2 * kGuard;
+        off += up256(dirs_plane_bytes(a.W, a.H));
+        k.E = scratch + vol_at[i];
+        k.W = a.W;
+        k.H = a.H;
+        k.D = a.D;
+        k.nd = paths == 8 ? 8 : 4;
+        k.vol = dirs_vol_bytes(a.W, a.H, a.D);
+        k.P1 = (uint32_t)p1h * 0x10001u;
+        k.P2 = (uint32_t)p2h * 0x10001u;
+        k.BIG = enc16(big) * 0x10001u;
+        k.BIG2 = enc16(2 * big) * 0x10001u;
+        k.err = (int*)(d_desc + out.ctl_off) + 1;
+        P.L = a.L;
+        P.R = a.R;
+        P.o.disp = a.disp;
+        P.o.disp_norm = a.disp_norm;
+        P.o.disp_right = a.disp_right;
+        P.o.lr_thr = a.lr_thr;
+        P.lr = a.lr_thr >= 0;
+        P.lpg = lanes_for(a.D);
+        P.prep_rows = std::max(1, kDirsPrepPixels / a.W);
+        P.nb[0] = (a.H + P.prep_rows - 1) / P.prep_rows;
+        switch (P.lpg) {
+            case 2: fill_lines<2, 1>(P); break;
+            case 4: fill_lines<4, 1>(P); break;
+            case 8: fill_lines<8, 1>(P); break;
+            case 16: fill_lines<16, 1>(P); break;
+            default: fill_lines<32, 2>(P); break;
+        }
+        // sum items: the consumer warps' lane groups over one or more rows,
+        // segments of at least 32 pixels
+        const int units = kBatchNW * 32 / P.lpg;
+        P.o.seglen = std::max(32, ((a.W + units - 1) / units + 7) & ~7);
+        P.o.nseg = (a.W + P.o.seglen - 1) / P.o.seglen;
+        P.o.rows = std::max(1, units / P.o.nseg);
+        while (P.o.rows > 1 && P.o.rows * a.W * 6 > 48 * 1024) P.o.rows--;
+        P.nb[2] = (a.H + P.o.rows - 1) / P.o.rows;
+        smem = std::max(smem, dirs_batch_smem(P.lpg));
+        sum_smem = std::max(sum_smem, kMaskBytes + P.o.rows * a.W * 6);
+    }
+    std::vector<DItem> items;
+    for (int i : idx)
+        for (int b = 0; b < hp[i].nb[0]; b++) items.push_back(DItem{i * 16, b});
+    out.launch_end.clear();
+    for (int w = 0; w < out.waves; w++)
+        for (int step = 1; step < kSteps; step++) {
+            for (int i : idx)
+                if (hp[i].wave == w)
+                    for (int b = 0; b < hp[i].nb[step]; b++) items.push_back(DItem{i * 16 + 2 * w + step, b});
+            out.launch_end.push_back((int)items.size());
+        }
+    out.dirs = paths == 8 ? 8 : 4;
+    out.n_pairs = n;
+    out.n_items = (int)items.size();
+    out.smem = smem;
+    out.sum_smem = sum_smem;
+    out.pairs_off = up256(sizeof(int) * (kDirsCtlHeader + (size_t)kSteps * n));
+    out.items_off = out.pairs_off + up256(sizeof(DPair) * n);
+    out.bytes = out.items_off + sizeof(DItem) * items.size();
+    out.item_bytes = (int)sizeof(DItem);
+    out.desc.assign(out.bytes, 0);
+    memcpy(out.desc.data() + out.pairs_off, hp.data(), sizeof(DPair) * n);
+    memcpy(out.desc.data() + out.items_off, items.data(), sizeof(DItem) * items.size());
+}
+
+namespace {
+
+template <int ND>
+cudaError_t configure_nd(const BatchPlan& plan) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(batch_dirs_kernel<ND, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(batch_dirs_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                plan.sum_smem);
+}
+
+template <int ND>
+cudaError_t launch_nd(const BatchPlan& plan, unsigned char* d_desc, unsigned long long wait_ns, int grid,
+                      cudaStream_t st, unsigned long long* trace) {
+    const DPair* pairs = (const DPair*)(d_desc + plan.pairs_off);
+    const DItem* items = (const DItem*)(d_desc + plan.items_off);
+    int* ctl = (int*)(d_desc + plan.ctl_off);
+    int first = 0;
+    for (size_t l = 0; l < plan.launch_end.size(); l++) {
+        const int last = plan.launch_end[l], head = 2 + (int)l;
+        if (l % 2 == 0)
+            batch_dirs_kernel<ND, false><<<3 * grid, kBatchT, plan.smem, st>>>(pairs, plan.n_pairs, items, first, last,
+                                                                               head, ctl, wait_ns, trace);
+        else
+            batch_dirs_kernel<ND, true><<<2 * grid, kBatchSumT, plan.sum_smem, st>>>(
+                pairs, plan.n_pairs, items, first, last, head, ctl, wait_ns, trace);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        first = last;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t batch_dirs_configure(const BatchPlan& plan) {
+    return plan.dirs == 8 ? configure_nd<8>(plan) : configure_nd<4>(plan);
+}
+
+cudaError_t batch_dirs_launch(const BatchPlan& plan, unsigned char* d_desc, unsigned long long wait_ns, int grid,
+                              cudaStream_t st, unsigned long long* trace) {
+    const cudaError_t e = cudaMemsetAsync(d_desc + plan.ctl_off, 0, plan.pairs_off - plan.ctl_off, st);
+    if (e != cudaSuccess) return e;
+    return plan.dirs == 8 ? launch_nd<8>(plan, d_desc, wait_ns, grid, st, trace)
+                          : launch_nd<4>(plan, d_desc, wait_ns, grid, st, trace);
 }
 
 }  // namespace tdv

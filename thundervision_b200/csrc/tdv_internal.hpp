@@ -353,6 +353,11 @@ struct BatchPlan {
     std::vector<unsigned char> desc;
     size_t ctl_off = 0, pairs_off = 0, items_off = 0, bytes = 0;
     int n_pairs = 0, n_items = 0, smem = 0, item_bytes = 0, ctas_per_sm = 1;
+    // directions stored apart: the paths (4 or 8, else 0), the waves, the end of
+    // each launch's items (lines and sums of one wave after another) and the
+    // sums' shared memory
+    int dirs = 0, waves = 0, sum_smem = 0;
+    std::vector<int> launch_end;
 };
 int batch_passes();
 int batch_threads();
@@ -363,7 +368,15 @@ size_t batch_scratch_bytes(const std::vector<BatchPairArgs>& pairs);
 // `d_desc` (device addresses, used only to fill pointers); returns an error
 // message, or nullptr on success.
 const char* batch_plan(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths,
-                       const BatchTiles& t, unsigned char* scratch, unsigned char* d_desc, BatchPlan& out);
+                       const BatchTiles& t, bool dirs, unsigned char* scratch, unsigned char* d_desc, BatchPlan& out);
+// The same batch with every direction stored apart (kernels_dirs.cu): scratch
+// of batch_dirs_scratch_bytes() (0: a pair or the penalties leave its range).
+size_t batch_dirs_scratch_bytes(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths);
+void batch_dirs_plan(const std::vector<BatchPairArgs>& pairs, int p1h, int p2h, int paths, bool longest_first,
+                     unsigned char* scratch, unsigned char* d_desc, BatchPlan& out);
+cudaError_t batch_dirs_configure(const BatchPlan& plan);
+cudaError_t batch_dirs_launch(const BatchPlan& plan, unsigned char* d_desc, unsigned long long wait_ns, int grid,
+                              cudaStream_t st, unsigned long long* trace);
 // Opts the persistent kernel into the plan's dynamic shared memory.
 cudaError_t batch_configure(const BatchPlan& plan);
 // Zeroes the control words and launches the persistent kernel (grid blocks);

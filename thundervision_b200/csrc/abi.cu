@@ -83,13 +83,24 @@ void release_buf(tdv_ctx* ctx, tdv_ctx::Buf& b) {
 
 cudaStream_t S(tdv_stream s) { return (cudaStream_t)s; }
 
-// Scratch of the directions stored apart, where the allocator has room for it:
-// false sends the call to the accumulating passes, which need a quarter to a
-// half of it.
-bool dirs_ready(tdv_ctx* ctx, tdv_ctx::Buf& b, int W, int H, int D, int paths, int excl) {
+// A capturing stream: allocating would invalidate the capture, so scratch that
+// a call can do without is left as earlier calls made it.
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return c != cudaStreamCaptureStatusNone;
+}
+
+// Scratch of the directions stored apart, where the allocator has room for it
+// (or an earlier call had, if the stream is capturing): false sends the call
+// to the accumulating passes, which need a quarter to a half of it.
+bool dirs_ready(tdv_ctx* ctx, tdv_ctx::Buf& b, int W, int H, int D, int paths, int excl, bool may_alloc) {
     const size_t n = tdv::dirs_bytes(W, H, D, paths, excl);
     if (b.bytes >= n) return true;
-    if (n >= ctx->dirs_refused) return false;
+    if (!may_alloc || n >= ctx->dirs_refused) return false;
     if (ensure(ctx, b, n) == TDV_OK) return true;
     ctx->dirs_refused = n;
     return false;
@@ -187,14 +198,15 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
 // of its own: all of them while their volumes stay within 10 GB, else four (a
 // group then also reads and writes S once, 8 bytes per cell beside 48); 0 where
 // the allocator has no room for them (the passes then run in sequence on S).
-int side_by_side(tdv_ctx* ctx, int W, int H, int D) {
+// A capturing call takes what is there.
+int side_by_side(tdv_ctx* ctx, int W, int H, int D, bool may_alloc) {
     const size_t vol = tdv::sgm_dirs_volume(W, H, D);
     const int np = (int)ctx->sched.passes.size();
     const int all = std::min(np, tdv::kMaxSideBySide);
     for (int g : {all * vol <= (size_t)10000000000 ? all : std::min(all, 4), std::min(all, 2)}) {
         const size_t need = g * vol;
         if (ctx->sgm_part.bytes >= need) return g;
-        if (need >= ctx->sgm_part_refused) continue;
+        if (!may_alloc || need >= ctx->sgm_part_refused) continue;
         if (ensure(ctx, ctx->sgm_part, need) == TDV_OK) return g;
         ctx->sgm_part_refused = need;
     }
@@ -217,14 +229,14 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     a.p2_adjust = p->p2_mode == TDV_P2_ADJUST;
     a.sem = p->semantics;
     const bool lr = out->lr_threshold >= 0 || out->disp_right;
-    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D) : 0;
+    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, !capturing(st)) : 0;
     const bool keep = aggreg || lr;  // the aggregated volume itself is needed
     VolArg Sv;
     if (aggreg) {
         Sv = tdv::make_vol(*aggreg);
     } else {
-        if (!group || keep || group < (int)ctx->sched.passes.size())
-            TDV_TRY(ensure(ctx, ctx->agg, (size_t)W * H * D * sizeof(float)));
+        // whether this call needs it or not: a later captured one may
+        TDV_TRY(ensure(ctx, ctx->agg, (size_t)W * H * D * sizeof(float)));
         tdv_volume tmp = *cost;
         tmp.ptr = ctx->agg.ptr;
         tmp.dtype = TDV_F32;  // the aggregation is float whatever the cost's type
@@ -576,7 +588,7 @@ tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t W, int32_t H, int32_t D) {
         return fail(ctx, TDV_ERR_INVALID_ARG, "bad reserve size %dx%dx%d", W, H, D);
     auto reserve = [&]() -> tdv_status {
         TDV_TRY(reserve_fused(ctx, W, H, D));
-        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1);
+        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, true);
         return TDV_OK;
     };
     if (!ctx->alloc) {
@@ -949,9 +961,14 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         fused = fused_weights_ready(ctx, W, H, D, params, fp, S(stream), &werr);
         TDV_TRY(werr);
     }
+    // the accumulating passes' scratch first, whichever path runs: a later
+    // captured call with other penalties may need it and cannot allocate
+    if (fused) {
+        TDV_TRY(reserve_fused(ctx, W, H, D));
+        TDV_TRY(ensure_side(ctx));
+    }
     if (fused && tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
-        dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl)) {
-        TDV_TRY(ensure(ctx, ctx->planes, tdv::dirs_plane_bytes(W, H)));
+        dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, !capturing(S(stream)))) {
         TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
         a.planes = ctx->planes.ptr;
@@ -960,8 +977,6 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         return TDV_OK;
     }
     if (fused) {
-        TDV_TRY(reserve_fused(ctx, W, H, D));
-        TDV_TRY(ensure_side(ctx));
         TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
         a.planes = ctx->planes.ptr;
@@ -1020,24 +1035,21 @@ tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left,
         if (!ok)
             return fail(ctx, TDV_ERR_UNSUPPORTED, "this size, table and semantics leave the fused path's ranges");
     }
-    const bool dirs = tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
-                      dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl) &&
-                      (n == 1 || dirs_ready(ctx, ctx->dirs_b, W, H, D, params->paths, fp.excl));
-    if (dirs) {
-        TDV_TRY(ensure(ctx, ctx->planes, tdv::dirs_plane_bytes(W, H)));
-    } else {
-        TDV_TRY(reserve_fused(ctx, W, H, D));
-        TDV_TRY(ensure_side(ctx));
-    }
+    TDV_TRY(reserve_fused(ctx, W, H, D));
+    TDV_TRY(ensure_side(ctx));
     TDV_TRY(ensure_err(ctx, st));
     if (n > 1) {
         TDV_TRY(ensure_lane(ctx));
-        TDV_TRY(ensure(ctx, ctx->planes_b, dirs ? tdv::dirs_plane_bytes(W, H) : tdv::fused_plane_bytes(W, H)));
-        if (!dirs) {
-            TDV_TRY(ensure(ctx, ctx->agg_b, tdv::fused_agg_bytes(W, H, D)));
-            TDV_TRY(ensure(ctx, ctx->agg2_b, tdv::fused_agg_bytes(W, H, D)));
-            if (fp.weighted && ctx->fside.bytes) TDV_TRY(ensure(ctx, ctx->fside_b, ctx->fside.bytes));
-        }
+        TDV_TRY(ensure(ctx, ctx->planes_b, std::max(tdv::fused_plane_bytes(W, H), tdv::dirs_plane_bytes(W, H))));
+        TDV_TRY(ensure(ctx, ctx->agg_b, tdv::fused_agg_bytes(W, H, D)));
+        TDV_TRY(ensure(ctx, ctx->agg2_b, tdv::fused_agg_bytes(W, H, D)));
+        if (fp.weighted && ctx->fside.bytes) TDV_TRY(ensure(ctx, ctx->fside_b, ctx->fside.bytes));
+    }
+    const bool may = !capturing(st);
+    const bool dirs = tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
+                      dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, may) &&
+                      (n == 1 || dirs_ready(ctx, ctx->dirs_b, W, H, D, params->paths, fp.excl, may));
+    if (n > 1) {
         // the second lane starts after what the call's stream holds
         TDV_CUDA(cudaEventRecord(ctx->lane_start, st));
         TDV_CUDA(cudaStreamWaitEvent(ctx->lane_main, ctx->lane_start, 0));

@@ -405,38 +405,41 @@ def _event_ms(fn, reps, warm, st):
     return e0.elapsed_time(e1) / reps
 
 
-def batch_trace_summary(tr, shapes, per_sm):
-    """Where one persistent batch run spends its block-time, from the per-item
-    trace (taken, dependency met, ended, smid << 32 | pair * 16 + pass): work,
-    dependency waits (per pass), the gaps a block spends between items, and
-    the tail each SM idles after its last item (per_sm blocks per SM take
-    items in turn; the tail is counted per SM); the time of the items of the
-    pairs below 0.25 Mpixel."""
+def batch_trace_summary(tr, shapes):
+    """Where one batch run (directions stored apart) spends its block-time,
+    from the per-item trace (taken, dependency met, ended, smid << 32 |
+    pair * 16 + pass): pass 0 prepares planes, 1 + 2w walks the lines of wave w
+    in the same launch as the planes (w = 0) and 2 + 2w sums it.  Every launch
+    is persistent, three blocks per SM for lines and two for sums: work,
+    dependency waits and the rest (launch start and tail), per kind and in all;
+    the share of the work that pairs below 0.25 Mpixel take."""
     import numpy as np
     t = tr.numpy().astype(np.int64)
     take, go, end = t[:, 0], t[:, 1], t[:, 2]
     ok = (take > 0) & (go >= take) & (end >= go)
     take, go, end, info = take[ok], go[ok], end[ok], t[ok, 3]
-    sm = info >> 32
+    sms = len(np.unique(info >> 32))
     pp = info & 0xFFFFFFFF
     pair, ps = pp >> 4, pp & 15
-    t0, t1 = take.min(), end.max()
-    span = float(t1 - t0)
-    slots = len(np.unique(sm)) * per_sm
-    busy = float((end - go).sum())
-    wait = float((go - take).sum())
-    last_end = {}
-    for s_, e_ in zip(sm, end):
-        last_end[s_] = max(last_end.get(s_, 0), e_)
-    tail = float(sum(t1 - e for e in last_end.values())) * per_sm
-    total = span * slots
+    launch = np.where(ps == 0, 1, ps)
+    kinds = {"lines": [0.0, 0.0, 0.0, 0.0], "sums": [0.0, 0.0, 0.0, 0.0]}
+    for n in np.unique(launch):
+        at = launch == n
+        span = float(end[at].max() - take[at].min())
+        k = kinds["lines" if n & 1 else "sums"]
+        for q, v in enumerate((span, span * sms * (3 if n & 1 else 2), float((end - go)[at].sum()),
+                               float((go - take)[at].sum()))):
+            k[q] += v
     small = np.array([w * h < 250000 for (w, h, d) in shapes])[pair]
-    names = ["prep", "V+", "V-", "D1+", "D1-", "D2+", "D2-", "H+", "H-"]
-    return {"span_ms": span / 1e6, "block_slots": int(slots),
-            "work_frac": busy / total, "dependency_wait_frac": wait / total, "tail_idle_frac": tail / total,
-            "other_frac": max(0.0, 1.0 - (busy + wait + tail) / total),
-            "wait_ms_by_pass": {names[p]: float((go - take)[ps == p].sum()) / 1e6 for p in range(9)},
-            "small_pairs_work_frac": float((end - go)[small].sum()) / max(busy, 1.0)}
+    busy, wait = (sum(k[q] for k in kinds.values()) for q in (2, 3))
+    total = sum(k[1] for k in kinds.values())
+    out = {"span_ms": float(end.max() - take.min()) / 1e6, "launches": int(len(np.unique(launch))),
+           "work_frac": busy / total, "dependency_wait_frac": wait / total, "rest_frac": 1.0 - (busy + wait) / total,
+           "small_pairs_work_frac": float((end - go)[small].sum()) / max(busy, 1.0)}
+    for name, k in kinds.items():
+        out[name] = {"span_ms": k[0] / 1e6, "work_frac": k[2] / max(k[1], 1.0),
+                     "dependency_wait_frac": k[3] / max(k[1], 1.0)}
+    return out
 
 
 def measure_batch(ctx, dev, reps=3):
@@ -457,12 +460,12 @@ def measure_batch(ctx, dev, reps=3):
         l, r, _, _ = synthetic.pair_sized(w, h, d, synthetic.pair_seed(0, i) % (2 ** 31))
         pairs.append((torch.from_numpy(l).to(dev), torch.from_numpy(r).to(dev), d))
     cells = sum(w * h * d * 8 for (w, h, d) in shapes)
-    # algorithmic bytes of the fused kernels: each pair's 16-bit volume holds
-    # 64 * ceil-to-{1,2,4}(D / 64) disparities per pixel and is touched 14 times
-    # (two first stores, four read-modify-writes, the join's two reads and one
-    # write, the last pass's read), plus the BT planes (34 B per pixel) per pass
-    span = lambda d: 64 if d <= 64 else (128 if d <= 128 else 256)
-    batch_bytes = sum(w * h * (2 * span(d) * 14 + 34 * 8) for (w, h, d) in shapes)
+    # algorithmic bytes of the kernels: eight byte volumes of the next power of
+    # two (16 at least) disparities per pixel, written once and read once; the
+    # BT planes (32 B per pixel) written once and read by lines and sum, and the
+    # images and the map
+    span = lambda d: max(16, 1 << (d - 1).bit_length())
+    batch_bytes = sum(w * h * (16 * span(d) + 3 * 32 + 4) for (w, h, d) in shapes)
     peak = 6650.0
     try:
         peak = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"]
@@ -514,7 +517,7 @@ def measure_batch(ctx, dev, reps=3):
     b.status()
     equal = all(torch.equal(o["disp"], ref) for o, ref in zip(b.outputs, fused_ref))
     n_items = b.work_queue()[1]
-    trace = batch_trace_summary(b.trace(), shapes, int(tiles.get("ctas_per_sm", 1)) if isinstance(tiles, dict) else 1)
+    trace = batch_trace_summary(b.trace(), shapes)
     b.close()
     return {"workload": "64 pairs, W~U[320,1920], H~U[240,1080] (x16), D in {32,64,128,256}, "
                         "BT + SGM-8 + WTA, seed 0",

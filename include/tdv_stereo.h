@@ -210,12 +210,12 @@ tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left,
 tdv_status tdv_stereo_sgm_static(const tdv_image* left, const tdv_image* right, int32_t max_disp,
                                  const tdv_sgm_params* params, tdv_disparity* out, tdv_stream stream);
 
-/* ---- batched pairs: one persistent launch (no reference counterpart) ----
+/* ---- batched pairs: one work queue (no reference counterpart) ----
  * The reference matches one pair per pipeline update
  * (tdvision/devstereomatcher.cpp:36-48 chains the cost and optimizer stages
  * of one frame); these calls run the fused integer-domain path of
- * tdv_stereo_sgm over many pairs of uneven size and disparity range in one
- * persistent kernel fed by a device work queue, with results bit-identical
+ * tdv_stereo_sgm over many pairs of uneven size and disparity range from a
+ * device work queue taken by persistent blocks, with results bit-identical
  * to per-pair tdv_stereo_sgm calls. */
 typedef struct {
     tdv_image left, right; /* TDV_U8, scale 1, device memory, equal sizes */
@@ -225,7 +225,8 @@ typedef struct {
 
 typedef enum { TDV_BATCH_ORDER_LONGEST_FIRST = 0, TDV_BATCH_ORDER_INPUT = 1 } tdv_batch_order;
 
-/* Tile shapes of the persistent kernel. */
+/* Tile shapes of the accumulating kernel.  Batches that store the directions
+ * apart (P1, P2 <= 127.5 and room for their volumes) take only `order`. */
 typedef struct {
     int32_t lines_per_cta;   /* vertical/diagonal passes: path lines per block, 1..24 */
     int32_t rows_per_cta;    /* horizontal passes: image rows per block, 1..25 (12 when split) */
@@ -255,7 +256,9 @@ tdv_status tdv_batch_get_tiles(const tdv_batch* batch, tdv_batch_tiles* tiles);
  * with its milliseconds per run. */
 tdv_status tdv_batch_autotune(tdv_batch* batch, int32_t reps, tdv_stream stream,
                               tdv_batch_tiles* chosen, double* best_ms);
-/* One run: zero the queue's control words, one persistent launch. */
+/* One run: zero the queue's control words, then one persistent launch, or one
+ * of lines and one of sums for each wave of pairs where the directions are
+ * stored apart. */
 tdv_status tdv_batch_run(tdv_batch* batch, tdv_stream stream);
 /* The same run through a CUDA graph, captured on first use (and again after
  * the tiles change) and replayed on `stream`. */
@@ -430,11 +433,13 @@ void tdv_ctx_destroy(tdv_ctx* ctx);
 tdv_status tdv_ctx_set_allocator(tdv_ctx* ctx, tdv_alloc_fn alloc, tdv_free_fn release,
                                  void* user);
 /* Pre-sizes the scratch of tdv_stereo_sgm (the fused path: planes, both
- * 16-bit aggregation volumes, the row scratch) for pairs up to W x H x D, so
- * later calls of it do not allocate.  The general path sizes its own scratch
- * on first use, once per size: tdv_sgm without a caller aggregation volume
- * (W x H x D floats, the path schedule, the deferred costs of repeated
- * walks), tdv_dp_scanline (W x H x D choice bytes), the filter-then-cost
+ * 16-bit aggregation volumes, the row scratch, and where the allocator has
+ * room the eight byte volumes of the directions stored apart) for pairs up to
+ * W x H x D, so later calls of it do not allocate.  The general path sizes its
+ * own scratch on first use, once per size: tdv_sgm (up to eight volumes of W x H x D
+ * floats while they fit 10 GB, four or two of them or none where the allocator
+ * refuses; the aggregation volume, the path schedule, the deferred costs of
+ * repeated walks), tdv_dp_scanline (W x H x D choice bytes), the filter-then-cost
  * case of tdv_cost_filtered (both filtered images).  A caller that must not
  * allocate later makes one call of each kind first, or passes its own
  * volumes. */
@@ -450,9 +455,9 @@ tdv_status tdv_ctx_device_status(tdv_ctx* ctx, tdv_stream stream);
  * most recent call and tdv_ctx_timing_name its kernel name.  This replaces the
  * reference's CudaBenchmarker around each stage update
  * (tdvision/benchmark.cpp:7-31, matchingcost.cpp:35-42).  While timing is on,
- * work a call would run concurrently on two streams (the fused 8-path pass
- * chains) runs in sequence on the call's stream, so each kernel is timed
- * alone. */
+ * work a call would run concurrently on two streams (the pass chains of the
+ * accumulating fused path) runs in sequence on the call's stream, so each
+ * kernel is timed alone. */
 tdv_status tdv_ctx_enable_timing(tdv_ctx* ctx, int32_t enable);
 int32_t tdv_ctx_timings(tdv_ctx* ctx, float* ms_out, int32_t max_entries);
 const char* tdv_ctx_timing_name(const tdv_ctx* ctx, int32_t index);

@@ -386,8 +386,8 @@ class Context:
 
 
 class Batch:
-    """Many uint8 pairs of uneven size and disparity range aggregated by one
-    persistent launch (tdv_batch_*): BT + SGM + WTA (+ left-right check) with
+    """Many uint8 pairs of uneven size and disparity range aggregated from
+    one device work queue (tdv_batch_*): BT + SGM + WTA (+ left-right check) with
     results bit-identical to per-pair ``Context.stereo_sgm`` calls.
 
     ``pairs`` is a list of ``(left, right, max_disp)`` or
@@ -431,7 +431,7 @@ class Batch:
             pass
 
     def run(self):
-        """One persistent launch on torch's current stream."""
+        """One run of the work queue on torch's current stream."""
         self.ctx.check(L.lib().tdv_batch_run(self.handle, _stream()))
         return self.outputs
 

@@ -1,5 +1,7 @@
 // Batched fused stereo: many integer-domain pairs of uneven size and
-// disparity range aggregated by ONE persistent launch.
+// disparity range aggregated by ONE persistent launch.  Batches whose pairs and
+// penalties allow the directions to be stored apart run batch_dirs_kernel
+// (kernels_dirs.cu) from the same kind of queue; this kernel is for the others.
 //
 // Work queue.  Every pass of every pair is cut into work items -- a band of
 // rows for the BT-plane prep, a group of G path lines for a vertical or

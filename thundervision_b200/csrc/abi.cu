@@ -20,6 +20,8 @@ using tdv::VolArg;
 namespace {
 
 using tdv_abi::DeviceScope;
+using tdv_abi::device_alloc;
+using tdv_abi::device_free;
 using tdv_abi::ensure;
 using tdv_abi::fail;
 using tdv_abi::kMaxSide;
@@ -74,9 +76,7 @@ tdv_status check_params(tdv_ctx* ctx, const tdv_sgm_params* p) {
 }
 
 void release_buf(tdv_ctx* ctx, tdv_ctx::Buf& b) {
-    if (!b.ptr) return;
-    if (ctx->release) ctx->release(b.ptr, ctx->alloc_user);
-    else cudaFree(b.ptr);
+    device_free(ctx, b.ptr);
     b.ptr = nullptr;
     b.bytes = 0;
 }
@@ -94,16 +94,50 @@ bool capturing(cudaStream_t st) {
     return c != cudaStreamCaptureStatusNone;
 }
 
+// Outgrown buffers that graphs hold: at most this much per context.
+constexpr size_t kMaxRetired = (size_t)10000000000;
+
+// Grows scratch a call can do without; a refusal leaves the buffer as it was.
+// The new buffer comes first, then the old one goes: set aside if a graph
+// holds its address, else freed once queued work is through with it.
+bool grow_optional(tdv_ctx* ctx, tdv_ctx::OptBuf& b, size_t bytes) {
+    if (b.bytes >= bytes) return true;
+    if (b.pinned && ctx->retired_bytes + b.bytes > kMaxRetired) return false;
+    void* p = device_alloc(ctx, bytes);
+    if (!p) return false;
+    if (b.pinned) {
+        ctx->retired.push_back(b);
+        ctx->retired_bytes += b.bytes;
+    } else if (b.ptr) {
+        cudaDeviceSynchronize();
+        device_free(ctx, b.ptr);
+    }
+    b.ptr = p;
+    b.bytes = bytes;
+    b.pinned = false;
+    return true;
+}
+
 // Scratch of the directions stored apart, where the allocator has room for it
 // (or an earlier call had, if the stream is capturing): false sends the call
-// to the accumulating passes, which need a quarter to a half of it.
-bool dirs_ready(tdv_ctx* ctx, tdv_ctx::Buf& b, int W, int H, int D, int paths, int excl, bool may_alloc) {
-    const size_t n = tdv::dirs_bytes(W, H, D, paths, excl);
-    if (b.bytes >= n) return true;
-    if (!may_alloc || n >= ctx->dirs_refused) return false;
-    if (ensure(ctx, b, n) == TDV_OK) return true;
-    ctx->dirs_refused = n;
-    return false;
+// to the accumulating passes, which need a quarter to a half of it.  It is
+// sized like the accumulation volumes, by W x H and the class of D alone (8
+// paths, the CPU recurrence's words), so that it grows only where they do; by
+// this call's own need where that is refused.
+bool dirs_ready(tdv_ctx* ctx, tdv_ctx::OptBuf& b, int W, int H, int D, int paths, int excl, bool captured) {
+    const size_t need = tdv::dirs_bytes(W, H, D, paths, excl);
+    if (b.bytes < need) {
+        if (captured || need >= ctx->dirs_refused) return false;
+        const int dclass = (int)(tdv::fused_agg_bytes(1, 1, D) / sizeof(uint16_t));
+        const size_t all = tdv::dirs_bytes(W, H, dclass, 8, 1);
+        if ((all >= ctx->dirs_refused || !grow_optional(ctx, b, all)) &&
+            (all == need || !grow_optional(ctx, b, need))) {
+            ctx->dirs_refused = need;
+            return false;
+        }
+    }
+    b.pinned = b.pinned || captured;
+    return true;
 }
 
 // Scratch of the fused path for pairs up to W x H x D: planes and both
@@ -199,15 +233,18 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
 // group then also reads and writes S once, 8 bytes per cell beside 48); 0 where
 // the allocator has no room for them (the passes then run in sequence on S).
 // A capturing call takes what is there.
-int side_by_side(tdv_ctx* ctx, int W, int H, int D, bool may_alloc) {
+int side_by_side(tdv_ctx* ctx, int W, int H, int D, bool captured) {
     const size_t vol = tdv::sgm_dirs_volume(W, H, D);
     const int np = (int)ctx->sched.passes.size();
     const int all = std::min(np, tdv::kMaxSideBySide);
     for (int g : {all * vol <= (size_t)10000000000 ? all : std::min(all, 4), std::min(all, 2)}) {
         const size_t need = g * vol;
-        if (ctx->sgm_part.bytes >= need) return g;
-        if (!may_alloc || need >= ctx->sgm_part_refused) continue;
-        if (ensure(ctx, ctx->sgm_part, need) == TDV_OK) return g;
+        if (ctx->sgm_part.bytes >= need) {
+            ctx->sgm_part.pinned = ctx->sgm_part.pinned || captured;
+            return g;
+        }
+        if (captured || need >= ctx->sgm_part_refused) continue;
+        if (grow_optional(ctx, ctx->sgm_part, need)) return g;
         ctx->sgm_part_refused = need;
     }
     return 0;
@@ -229,7 +266,7 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     a.p2_adjust = p->p2_mode == TDV_P2_ADJUST;
     a.sem = p->semantics;
     const bool lr = out->lr_threshold >= 0 || out->disp_right;
-    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, !capturing(st)) : 0;
+    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, capturing(st)) : 0;
     const bool keep = aggreg || lr;  // the aggregated volume itself is needed
     VolArg Sv;
     if (aggreg) {
@@ -531,7 +568,7 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
                      ctx->misc.ptr || ctx->sched_buf.ptr || ctx->err.ptr || ctx->soft.ptr ||
                      ctx->agg2.ptr || ctx->defer.ptr || ctx->side || ctx->fw_buf.ptr || ctx->fside.ptr ||
                      ctx->lane_main || ctx->planes_b.ptr || ctx->agg_b.ptr || ctx->agg2_b.ptr || ctx->fside_b.ptr ||
-                     ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr;
+                     ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr || !ctx->retired.empty();
     if (any) {
         DeviceScope ds(ctx->device);
         cudaDeviceSynchronize();
@@ -557,6 +594,7 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
         release_buf(ctx, ctx->dirs);
         release_buf(ctx, ctx->dirs_b);
         release_buf(ctx, ctx->sgm_part);
+        for (tdv_ctx::Buf& b : ctx->retired) release_buf(ctx, b);
         if (ctx->lane_main) cudaStreamDestroy(ctx->lane_main);
         if (ctx->lane_side) cudaStreamDestroy(ctx->lane_side);
         for (cudaEvent_t e : {ctx->lane_fork, ctx->lane_join, ctx->lane_start, ctx->lane_done})
@@ -588,7 +626,7 @@ tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t W, int32_t H, int32_t D) {
         return fail(ctx, TDV_ERR_INVALID_ARG, "bad reserve size %dx%dx%d", W, H, D);
     auto reserve = [&]() -> tdv_status {
         TDV_TRY(reserve_fused(ctx, W, H, D));
-        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, true);
+        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, false);
         return TDV_OK;
     };
     if (!ctx->alloc) {
@@ -968,7 +1006,7 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         TDV_TRY(ensure_side(ctx));
     }
     if (fused && tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
-        dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, !capturing(S(stream)))) {
+        dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, capturing(S(stream)))) {
         TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
         a.planes = ctx->planes.ptr;
@@ -1045,10 +1083,10 @@ tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left,
         TDV_TRY(ensure(ctx, ctx->agg2_b, tdv::fused_agg_bytes(W, H, D)));
         if (fp.weighted && ctx->fside.bytes) TDV_TRY(ensure(ctx, ctx->fside_b, ctx->fside.bytes));
     }
-    const bool may = !capturing(st);
+    const bool captured = capturing(st);
     const bool dirs = tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
-                      dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, may) &&
-                      (n == 1 || dirs_ready(ctx, ctx->dirs_b, W, H, D, params->paths, fp.excl, may));
+                      dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, captured) &&
+                      (n == 1 || dirs_ready(ctx, ctx->dirs_b, W, H, D, params->paths, fp.excl, captured));
     if (n > 1) {
         // the second lane starts after what the call's stream holds
         TDV_CUDA(cudaEventRecord(ctx->lane_start, st));
@@ -1100,22 +1138,6 @@ struct tdv_batch {
 
 namespace {
 
-void* dev_alloc(tdv_ctx* ctx, size_t bytes) {
-    void* p = nullptr;
-    if (ctx->alloc) return ctx->alloc(bytes, ctx->alloc_user);
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return p;
-}
-
-void dev_free(tdv_ctx* ctx, void* p) {
-    if (!p) return;
-    if (ctx->release) ctx->release(p, ctx->alloc_user);
-    else cudaFree(p);
-}
-
 void drop_graph(tdv_batch* b) {
     if (b->gexec) cudaGraphExecDestroy(b->gexec);
     b->gexec = nullptr;
@@ -1132,8 +1154,8 @@ tdv_status batch_replan(tdv_batch* b, const tdv_batch_tiles& t) {
         if (msg) return fail(ctx, TDV_ERR_UNSUPPORTED, "batch tiles: %s", msg);
         if (plan.bytes > b->desc_bytes) {
             // the descriptors hold the queue's own address: grow, then plan again
-            dev_free(ctx, b->desc);
-            b->desc = dev_alloc(ctx, plan.bytes);
+            device_free(ctx, b->desc);
+            b->desc = device_alloc(ctx, plan.bytes);
             b->desc_bytes = b->desc ? plan.bytes : 0;
             if (!b->desc) return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of work queue failed", plan.bytes);
             continue;
@@ -1213,10 +1235,10 @@ tdv_status tdv_batch_create(tdv_ctx* ctx, const tdv_batch_pair* pairs, int32_t n
     }
     // every direction stored apart where the range and the memory allow
     const size_t db = tdv::batch_dirs_scratch_bytes(b->pairs, b->p1h, b->p2h, b->paths);
-    if (db) b->scratch = dev_alloc(ctx, db);
+    if (db) b->scratch = device_alloc(ctx, db);
     b->dirs = b->scratch != nullptr;
     const size_t sb = tdv::batch_scratch_bytes(b->pairs);
-    if (!b->dirs) b->scratch = dev_alloc(ctx, sb);
+    if (!b->dirs) b->scratch = device_alloc(ctx, sb);
     if (!b->scratch) {
         delete b;
         return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of batch scratch failed", sb);
@@ -1241,8 +1263,8 @@ void tdv_batch_destroy(tdv_batch* b) {
     DeviceScope ds(b->ctx->device);
     cudaDeviceSynchronize();
     drop_graph(b);
-    dev_free(b->ctx, b->scratch);
-    dev_free(b->ctx, b->desc);
+    device_free(b->ctx, b->scratch);
+    device_free(b->ctx, b->desc);
     delete b;
 }
 

@@ -44,6 +44,23 @@ struct DeviceScope {
     }
 };
 
+// Device memory from the caller's allocator, or the driver's; null if refused.
+inline void* device_alloc(tdv_ctx* ctx, size_t bytes) {
+    if (ctx->alloc) return ctx->alloc(bytes, ctx->alloc_user);
+    void* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return p;
+}
+
+inline void device_free(tdv_ctx* ctx, void* p) {
+    if (!p) return;
+    if (ctx->release) ctx->release(p, ctx->alloc_user);
+    else cudaFree(p);
+}
+
 // Scratch buffers grow on demand; growing waits for the device first because
 // work already queued may still read the old buffer.
 inline tdv_status ensure(tdv_ctx* ctx, tdv_ctx::Buf& b, size_t bytes) {
@@ -51,18 +68,11 @@ inline tdv_status ensure(tdv_ctx* ctx, tdv_ctx::Buf& b, size_t bytes) {
     if (b.bytes >= bytes) return TDV_OK;
     if (b.ptr) {
         cudaDeviceSynchronize();
-        if (ctx->release) ctx->release(b.ptr, ctx->alloc_user);
-        else cudaFree(b.ptr);
+        device_free(ctx, b.ptr);
         b.ptr = nullptr;
         b.bytes = 0;
     }
-    void* p = nullptr;
-    if (ctx->alloc) {
-        p = ctx->alloc(bytes, ctx->alloc_user);
-    } else if (cudaMalloc(&p, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        p = nullptr;
-    }
+    void* p = device_alloc(ctx, bytes);
     if (!p) return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of scratch failed", bytes);
     b.ptr = p;
     b.bytes = bytes;

@@ -168,6 +168,12 @@ struct tdv_ctx {
         void* ptr = nullptr;
         size_t bytes = 0;
     };
+    // Scratch a call can do without.  A captured call's graph keeps the address
+    // it was given, so a buffer that a capturing call used (`pinned`) is never
+    // freed before the context: growth sets it aside in `retired`.
+    struct OptBuf : Buf {
+        bool pinned = false;
+    };
     Buf agg;      // aggregation volume
     Buf agg2;     // fused path: second aggregation volume (concurrent pass chains)
     Buf cost;     // cost DSI for tdv_stereo_sgm's general path
@@ -197,11 +203,13 @@ struct tdv_ctx {
     // fused path with the directions stored apart (kernels_dirs.cu), per lane;
     // dirs_refused: the smallest such request the allocator turned down, so
     // that later calls of that size go straight to the accumulating passes
-    Buf dirs, dirs_b;
+    OptBuf dirs, dirs_b;
     size_t dirs_refused = (size_t)-1;
     // general path with the passes side by side (kernels_sgm_dirs.cu)
-    Buf sgm_part;
+    OptBuf sgm_part;
     size_t sgm_part_refused = (size_t)-1;
+    std::vector<Buf> retired;   // pinned buffers that were outgrown
+    size_t retired_bytes = 0;
     cudaStream_t lane_main = nullptr, lane_side = nullptr;
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr, lane_start = nullptr, lane_done = nullptr;
 };

@@ -22,8 +22,11 @@
 // A lane owns 8 consecutive disparities and a walk takes 4 to 32 lanes, so a
 // warp runs up to 8 walks (one walk per warp with lane-interleaved disparities
 // spends two shuffles per register and step, and all its per-step work on 64
-// disparities); C and L move as 32-byte accesses where runs are aligned, and
-// the C loads run ahead in a register ring.
+// disparities); C moves as 32-byte accesses where runs are aligned, and its
+// loads run ahead in a register ring.  The runs of L are padded to a multiple
+// of 8 disparities, so L always does: eight 4-byte stores per lane at a stride
+// of 32 bytes instead took D = 127 at 1920x1080 from 6.3 ms in sequence to 7.9,
+// and D = 60 at 3840x2160 from 11.0 to 17.8; padded they take 5.2 and 10.2.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -64,9 +67,9 @@ __device__ __forceinline__ uint32_t ford(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-// A lane's 8 consecutive elements at p.  VEC: D is a multiple of 8 and both
-// volumes start on 32 bytes, so a lane's elements are all inside the run or
-// all outside and move as one 32-byte access (16 bytes for a 16-bit cost).
+// A lane's 8 consecutive costs at p.  VEC: D is a multiple of 8 and the volume
+// starts on 32 bytes, so a lane's elements are all inside the run or all
+// outside and move as one 32-byte access (16 bytes for a 16-bit cost).
 template <bool VEC>
 __device__ __forceinline__ void load_run(const float* p, int n, float* v) {
     if constexpr (VEC) {
@@ -97,18 +100,12 @@ __device__ __forceinline__ void load_run(const uint16_t* p, int n, uint16_t* v) 
         for (int j = 0; j < 8; j++) v[j] = j < n ? p[j] : (uint16_t)0xFFFFu;
     }
 }
-template <bool VEC>
+// A lane's 8 path costs (what lies past D is padding).
 __device__ __forceinline__ void store_run(float* p, int n, const float* v) {
-    if constexpr (VEC) {
-        if (n > 0)
-            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
-                         "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                         : "memory");
-    } else {
-#pragma unroll
-        for (int j = 0; j < 8; j++)
-            if (j < n) p[j] = v[j];
-    }
+    if (n > 0)
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
+                     "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                     : "memory");
 }
 
 // Minimum over a walk's disparities (nm of this lane's eight count) with
@@ -153,7 +150,11 @@ __global__ void __launch_bounds__(128) sgm_dirs_kernel(SgmArgs a, const Walk* __
     const int nm = refcpu ? nd - 1 : nd;      // REF_CPU scans {sentinel, L(0..D-2)}
     const long long off = wk.sx * a.C.sx + wk.sy * a.C.sy + d0, stride = dx * a.C.sx + dy * a.C.sy;
     const CT* cq = (const CT*)a.C.ptr + off;
-    float* lq = part + pi * vol + off;
+    // the path costs' runs are padded to whole lanes: always one 32-byte store
+    const int Dp = (D + 7) & ~7;
+    const long long px = a.C.sx / D, py = a.C.sy / D;  // pixels
+    float* lq = part + pi * vol + (wk.sx * px + wk.sy * py) * Dp + d0;
+    const long long lstride = (dx * px + dy * py) * Dp;
     const int len = wk.len;
     const int steps = __reduce_max_sync(FULLM, len);
     constexpr int K = 4;  // steps of C in flight (two: 0.275 ms against 0.220 at 640x480, D = 64)
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(128) sgm_dirs_kernel(SgmArgs a, const Walk* __
         load_run<VEC>(cq, 1 + i < len ? nd : 0, ring[i]);
         cq += stride;
     }
-    store_run<VEC>(lq, len > 0 ? nd : 0, L);
+    store_run(lq, len > 0 ? nd : 0, L);
     float m = walk_min<LPG>(L, nm);
     if (refgpu) {
 #pragma unroll
@@ -228,10 +229,10 @@ __global__ void __launch_bounds__(128) sgm_dirs_kernel(SgmArgs a, const Walk* __
             }
             load_run<VEC>(cq, t0 + u + K < len ? nd : 0, ring[i]);
             cq += stride;
-            lq += stride;
+            lq += lstride;
 #pragma unroll
             for (int j = 0; j < 8; j++) L[j] = Ln[j];
-            store_run<VEC>(lq, t0 + u < len ? nd : 0, L);
+            store_run(lq, t0 + u < len ? nd : 0, L);
             m = walk_min<LPG>(L, nm);
         }
     }
@@ -248,7 +249,7 @@ struct SumArgs {
     const float* Sin;        // S of the groups before this one, or null
     float* S;                // S stored, or null
     const uint16_t* mult;    // per pass nl line counts (0: no walk, n: n times)
-    int nl, W, H, D, xmajor;
+    int nl, W, H, D, Dp, xmajor;
     int dx[kMaxSideBySide], dy[kMaxSideBySide];
     int first;               // the group's first pass writes S
     uint16_t* disp;          // winners, or null
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(256) sgm_sum_kernel(SumArgs a) {
     const int lane = threadIdx.x & 31;
     const uint32_t npix = (uint32_t)a.W * (uint32_t)a.H, side = a.xmajor ? a.H : a.W;
     for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < npix; q += (gridDim.x * blockDim.x) >> 5) {
-        const float* p = a.part + (size_t)q * a.D + lane;
+        const float* p = a.part + (size_t)q * a.Dp + lane;
         float v[N][NP], s[N];
 #pragma unroll
         for (int i = 0; i < N; i++)
@@ -351,7 +352,7 @@ cudaError_t run_group(const SgmArgs& a, const PassSchedule& sch, const DirGroup&
 template <typename CT>
 cudaError_t run_group_any(const SgmArgs& a, const PassSchedule& sch, const DirGroup& g, int blocks, int lpg, float* part,
                           size_t vol, cudaStream_t st) {
-    const bool vec = a.C.D % 8 == 0 && ((uintptr_t)a.C.ptr & 31) == 0 && ((uintptr_t)part & 31) == 0;
+    const bool vec = a.C.D % 8 == 0 && ((uintptr_t)a.C.ptr & 31) == 0;
     switch (lpg) {
         case 4: return vec ? run_group<4, CT, true>(a, sch, g, blocks, part, vol, st)
                            : run_group<4, CT, false>(a, sch, g, blocks, part, vol, st);
@@ -388,7 +389,10 @@ cudaError_t run_sum_np(const SumArgs& s, int np, bool plain, bool refcpu, int gr
 
 }  // namespace
 
-size_t sgm_dirs_volume(int W, int H, int D) { return ((size_t)W * H * D * sizeof(float) + 255) & ~(size_t)255; }
+// Bytes of one pass's path costs, each run padded to a multiple of 8.
+size_t sgm_dirs_volume(int W, int H, int D) {
+    return ((size_t)W * H * ((D + 7) & ~7) * sizeof(float) + 255) & ~(size_t)255;
+}
 
 cudaError_t launch_sgm_dirs(const SgmArgs& a, const PassSchedule& sch, float* part, int group,
                             float* S, bool keep, uint16_t* disp, float* disp_norm, cudaStream_t st, Timer* tm) {
@@ -425,6 +429,7 @@ cudaError_t launch_sgm_dirs(const SgmArgs& a, const PassSchedule& sch, float* pa
         s.W = W;
         s.H = H;
         s.D = D;
+        s.Dp = (D + 7) & ~7;
         s.xmajor = a.C.sx > a.C.sy ? 1 : 0;
         s.first = g0 == 0;
         s.disp = disp;

@@ -266,7 +266,7 @@ struct SgmArgs {
     float* defer;  // path costs of the repeated walks of one pass (PassSchedule::defer_rows x D)
 };
 // The passes side by side in groups of `group` volumes (at most
-// kMaxSideBySide) at `part`, sgm_dirs_volume() bytes each: S is stored when
+// kMaxSideBySide) at `part` (on 32 bytes), sgm_dirs_volume() bytes each: S is stored when
 // `keep` (and between groups), the winners always.  Needs sch.lines.
 constexpr int kMaxSideBySide = 8;
 size_t sgm_dirs_volume(int W, int H, int D);

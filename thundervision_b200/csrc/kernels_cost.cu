@@ -1,7 +1,7 @@
 // Matching-cost DSI writers, banded: Birchfield-Tomasi (tdvision/birchfieldcost.cu:14-59),
 // window SSD (ssd.cu:15-50) and un-centred NCC (crosscorrelation.cu:11-49).
 //
-// One CTA owns a tile of kTX x TY pixels (TY 4 or 8, see tall_tiles) and all D
+// One CTA owns a tile of kTX x TY pixels (TY 8, 4 or 2, see tile_rows) and all D
 // disparities of them.
 //   * Staging: the rows the tile's windows touch are read once, clamped to
 //     each image's own edges and multiplied by its scale exactly as the
@@ -45,6 +45,9 @@ constexpr int kTX = 64;           // tile width (pixels)
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxBandBytes = 220 * 1024;
+// columns the fused Gaussian of the window costs filters at a time
+constexpr int kFilterCols = 144;
+constexpr int kThreeBlocks = 75 * 1024, kTwoBlocks = 113 * 1024;  // shared memory of a block, so many to an SM
 
 __device__ __forceinline__ float fetch(const ImgArg& im, int x, int y) {
     x = min(max(x, 0), im.W - 1);
@@ -85,7 +88,10 @@ struct Band {
     // the raw rows with a 2-pixel halo and their row pass as scratch.
     __host__ __device__ static int fl_band(const Geom& g) { return floats(g); }
     __host__ __device__ static int fr_band(const Geom& g) { return fl_band(g) + TY * (kTX + 2); }
-    __host__ __device__ static int widest(const Geom& g) { return KIND == TDV_COST_BT ? kTX + g.D + 1 : g.rbw; }
+    __host__ __device__ static int widest(const Geom& g) {
+        if (KIND == TDV_COST_BT) return kTX + g.D + 1;
+        return g.rbw < kFilterCols ? g.rbw : kFilterCols;
+    }
     __host__ __device__ static int scratch(const Geom& g) {
         return KIND == TDV_COST_BT ? fr_band(g) + TY * (kTX + g.D + 1) : floats(g);
     }
@@ -148,36 +154,51 @@ __device__ __forceinline__ void bt_terms(const ImgArg& im, int x, int y, float& 
     ma = fmaxf(a, fmaxf(b, I));
 }
 
+// Where gauss_band puts a value: BT's band of samples, row by row (one type for
+// both images: two lambdas made two copies of the code, 87.4 us against 86.1 at
+// 640x480, D = 256).
+struct PlainBand {
+    float* b;
+    int w;
+    __device__ __forceinline__ void operator()(int row, int col, float v) const { b[row * w + col] = v; }
+};
+
 // put(row, col, G(clamp(c0 + col), clamp(r0 + row))) for the 5x5
 // Gaussian G of the image with replicated borders (the pre-filter kernel's
 // values, bit for bit): the raw rows the clamped range needs, with a 2-pixel
 // halo, then the row pass, then the column pass, in that kernel's order.
-template <typename Put>
+// CHUNKS: kFilterCols columns at a time, so that the scratch does not grow with
+// D (BT's band is small and takes all at once: the loop costs it 2 %).
+template <bool CHUNKS, typename Put>
 __device__ void gauss_band(const ImgArg& im, int c0, int ncols, int r0, int nrows, Put put, float* scratch) {
     const int tid = threadIdx.x;
-    const int c_lo = min(max(c0, 0), im.W - 1), c_hi = min(max(c0 + ncols - 1, 0), im.W - 1);
     const int r_lo = min(max(r0, 0), im.H - 1), r_hi = min(max(r0 + nrows - 1, 0), im.H - 1);
-    const int nc = c_hi - c_lo + 1, nr = r_hi - r_lo + 1;
-    float* raw = scratch;                   // [nr + 4][nc + 4]
-    float* rp = scratch + (nr + 4) * (nc + 4);  // [nr + 4][nc]
-    for (int i = tid; i < (nr + 4) * (nc + 4); i += kThreads) {
-        const int row = i / (nc + 4), col = i - row * (nc + 4);
-        raw[i] = fetch(im, c_lo - 2 + col, r_lo - 2 + row);
+    const int nr = r_hi - r_lo + 1;
+    for (int b = 0; b < ncols; b += CHUNKS ? kFilterCols : ncols) {
+        const int nb = CHUNKS ? min(ncols - b, kFilterCols) : ncols, cb = c0 + b;
+        const int c_lo = min(max(cb, 0), im.W - 1), c_hi = min(max(cb + nb - 1, 0), im.W - 1);
+        const int nc = c_hi - c_lo + 1;
+        float* raw = scratch;                       // [nr + 4][nc + 4]
+        float* rp = scratch + (nr + 4) * (nc + 4);  // [nr + 4][nc]
+        for (int i = tid; i < (nr + 4) * (nc + 4); i += kThreads) {
+            const int row = i / (nc + 4), col = i - row * (nc + 4);
+            raw[i] = fetch(im, c_lo - 2 + col, r_lo - 2 + row);
+        }
+        __syncthreads();
+        for (int i = tid; i < (nr + 4) * nc; i += kThreads) {
+            const int row = i / nc, col = i - row * nc;
+            const float* t = raw + row * (nc + 4) + col;
+            rp[i] = gauss5(t[0], t[1], t[2], t[3], t[4]);
+        }
+        __syncthreads();
+        for (int i = tid; i < nrows * nb; i += kThreads) {
+            const int row = i / nb, col = i - row * nb;
+            const int cc = min(max(cb + col, 0), im.W - 1) - c_lo, rr = min(max(r0 + row, 0), im.H - 1) - r_lo;
+            const float* t = rp + rr * nc + cc;
+            put(row, b + col, gauss5(t[0], t[nc], t[2 * nc], t[3 * nc], t[4 * nc]));
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    for (int i = tid; i < (nr + 4) * nc; i += kThreads) {
-        const int row = i / nc, col = i - row * nc;
-        const float* t = raw + row * (nc + 4) + col;
-        rp[i] = gauss5(t[0], t[1], t[2], t[3], t[4]);
-    }
-    __syncthreads();
-    for (int i = tid; i < nrows * ncols; i += kThreads) {
-        const int row = i / ncols, col = i - row * ncols;
-        const int cc = min(max(c0 + col, 0), im.W - 1) - c_lo, rr = min(max(r0 + row, 0), im.H - 1) - r_lo;
-        const float* t = rp + rr * nc + cc;
-        put(row, col, gauss5(t[0], t[nc], t[2 * nc], t[3 * nc], t[4 * nc]));
-    }
-    __syncthreads();
 }
 
 // BT terms from a band of (filtered) samples: b[0], b[1], b[2] are the
@@ -282,9 +303,8 @@ __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0,
         float* fl = sm + B::fl_band(g);     // [B::TY][kTX + 2]: columns x0 - 1 .. x0 + kTX
         float* fr = sm + B::fr_band(g);     // [B::TY][kTX + D + 1]: columns x0 - D .. x0 + kTX
         float* scr = sm + B::scratch(g);
-        gauss_band(L, x0 - 1, kTX + 2, y0, B::TY, [&](int r, int c, float v) { fl[r * (kTX + 2) + c] = v; }, scr);
-        gauss_band(Rim, x0 - g.D, kTX + g.D + 1, y0, B::TY,
-                   [&](int r, int c, float v) { fr[r * (kTX + g.D + 1) + c] = v; }, scr);
+        gauss_band<false>(L, x0 - 1, kTX + 2, y0, B::TY, PlainBand{fl, kTX + 2}, scr);
+        gauss_band<false>(Rim, x0 - g.D, kTX + g.D + 1, y0, B::TY, PlainBand{fr, kTX + g.D + 1}, scr);
         float* lt = sm;
         float* rt = sm + B::rband(g);
         for (int i = tid; i < kTX * B::TY; i += kThreads) {
@@ -312,9 +332,9 @@ __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0,
         float* lb = sm;
         float* rb = sm + B::rband(g);
         float* scr = sm + B::scratch(g);
-        gauss_band(L, x0 - R, kTX + 2 * R, y0 - R, B::kRows,
+        gauss_band<true>(L, x0 - R, kTX + 2 * R, y0 - R, B::kRows,
                    [&](int r, int c, float v) { B::put_left(lb + r * B::kLeft, c, v); }, scr);
-        gauss_band(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows,
+        gauss_band<true>(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows,
                    [&](int r, int c, float v) { B::put_right(rb + r * g.rbw * 2, c, v); }, scr);
         if (fl_out)
             for (int i = tid; i < kTX * B::TY; i += kThreads) {
@@ -341,7 +361,7 @@ __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0,
 // DSI writer, D = 64, ms before / pairs / pairs and two rows: 1920x1080 SSD 7x7
 // 0.456 / 0.396 / 0.319, NCC 9x9 0.732 / 0.669 / 0.603; 640x480 SSD 5x5 0.056 /
 // 0.049 / 0.040, NCC 9x9 0.127 / 0.119 / 0.110.
-template <int KIND, int R, int HP>
+template <int KIND, int R, int HP, int NR>
 __device__ __forceinline__ void window_sums(const f2* l, int lstride, const f2* r, int rstride, f2 nz,
                                             f2 (*acc)[HP]) {
     constexpr int NJ = HP + 2 * R;
@@ -374,20 +394,22 @@ __device__ __forceinline__ void window_sums(const f2* l, int lstride, const f2* 
             for (int p = 0; p < HP; p++) s[p] = add2(s[p], t[p + b]);
     };
 #pragma unroll
-    for (int p = 0; p < HP; p++) acc[0][p] = acc[1][p] = 0ull;
+    for (int p = 0; p < HP; p++) acc[0][p] = acc[NR - 1][p] = 0ull;
     taps();
     add_row(acc[0]);
 #pragma unroll 1
     for (int a = 1; a <= 2 * R; a++) {
         taps();
         add_row(acc[0]);
+        if (NR == 2) add_row(acc[1]);
+    }
+    if (NR == 2) {
+        taps();
         add_row(acc[1]);
     }
-    taps();
-    add_row(acc[1]);
 }
 
-template <int KIND, int R, int P, bool FILT, int TY>
+template <int KIND, int R, int P, bool FILT, int TY, int NR>
 __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Rim, VolArg out, Geom g,
                                                              int tiles_x, float* fl_out) {
     extern __shared__ __align__(16) float sm[];
@@ -403,7 +425,7 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
     const int span = P * g.G;                   // pixels of one work item
     const int groups = kTX / span;
     const int chunks = (D + g.Dw - 1) / g.Dw;
-    const int items = B::TY / 2 * groups * chunks;  // (SSD, NCC) two rows each
+    const int items = B::TY / NR * groups * chunks;  // (SSD, NCC) NR rows each
     float* const outp = (float*)out.ptr;
 
     if (KIND == TDV_COST_BT) {
@@ -478,18 +500,18 @@ __global__ void __launch_bounds__(kThreads) cost_band_kernel(ImgArg L, ImgArg Ri
         for (int it = warp; it < items; it += kWarps) {
             const int chunk = it % chunks;
             const int rest = it / chunks;
-            const int grp = rest % groups, row = 2 * (rest / groups);
+            const int grp = rest % groups, row = NR * (rest / groups);
             const int xs = x0 + grp * span + sub * P;   // first pixel of this thread
             const int d = chunk * g.Dw + dl;
             const bool dok = d < D;
             const int de = dok ? d : D - 1;             // lanes past D read in-band columns, store nothing
-            f2 acc[2][HP];
-            window_sums<KIND, R, HP>(
+            f2 acc[NR][HP];
+            window_sums<KIND, R, HP, NR>(
                 reinterpret_cast<const f2*>(sm) + row * (B::kLeft / 2) + (xs - x0) / P * B::kJ, B::kLeft / 2,
                 reinterpret_cast<const f2*>(sm + B::rband(g)) + row * g.rbw + (xs - de) - (x0 - (D - 1)), g.rbw, g.nz,
                 acc);
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < NR; i++) {
                 const int y = y0 + row + i;
                 float v[P];
 #pragma unroll
@@ -589,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, 3) fastwta_band_kernel(ImgArg L, Img
             const bool dok = d < D;
             const int de = dok ? d : D - 1;
             f2 sums[2][HP];
-            window_sums<TDV_COST_SSD, R, HP>(
+            window_sums<TDV_COST_SSD, R, HP, 2>(
                 reinterpret_cast<const f2*>(sm) + row * (B::kLeft / 2) + (xs - x0) / P * B::kJ, B::kLeft / 2,
                 reinterpret_cast<const f2*>(sm + B::rband(g)) + row * g.rbw + (xs - de) - (x0 - (D - 1)), g.rbw, g.nz,
                 sums);
@@ -634,18 +656,43 @@ __global__ void __launch_bounds__(kThreads, 3) fastwta_band_kernel(ImgArg L, Img
     }
 }
 
-// Tile height: 8 rows share a window's halo, its filter and its window sums
+// Tile height.  8 rows share a window's halo, its filter and its window sums
 // better, 4 spread a small image over the chip (NCC 9x9, D = 64: 0.603 / 0.620
 // ms at 1920x1080, 0.120 / 0.110 at 640x480; BT 0.125 / 0.132 and 0.029 /
-// 0.025): 8 from ten rounds of tiles over 148 SMs on.
-bool tall_tiles(int W, int H) { return (long long)((W + kTX - 1) / kTX) * ((H + 7) / 8) >= 1480; }
+// 0.025): 8 from ten rounds of tiles over 148 SMs on, and
+//   * only while three blocks of shared memory fit an SM (filtered NCC 9x9,
+//     1920x1080, D = 200: 97 KB a block, 2.19 ms against 2.04; filtered BT,
+//     1280x720, D = 256: 0.235 against 0.216);
+//   * for BT of long ranges from twenty rounds on (1280x720, D = 256: 0.182
+//     against 0.173; 1920x1080, D = 128: 0.202 against 0.208);
+//   * for SSD up to D = 16 always: a work item is then 32 or 64 pixels of two
+//     rows, and 4 rows leave half the block's warps without one (7x7 filtered,
+//     640x480, D = 8: 24 us against 34);
+//   * not for the 9x9 NCC up to D = 31 (1280x720, D = 16: 118 us against 112).
+// 2 rows where a block of 4 takes an SM for itself (NCC 3x3, D = 1900, 640x128:
+// 0.73 ms against 0.79 with 4); FastWTA keeps 4 there (it measured slower with
+// 2: 7x7, D = 1800, 0.89 ms against 0.75).
+template <int KIND, int R, int HP, bool FILT, int TY>
+int band_bytes(const Geom& g) {
+    using B = Band<KIND, R, HP, TY>;
+    return (FILT ? B::floats_filtered(g) : B::floats(g)) * 4;
+}
+template <int KIND, int R, int HP, bool FILT>
+int tile_rows(int W, int H, const Geom& g) {
+    const long long tiles = (long long)((W + kTX - 1) / kTX) * ((H + 7) / 8);
+    long long tall = 1480;
+    if (KIND == TDV_COST_BT && g.D > 100) tall = 2960;
+    if (KIND != TDV_COST_NCC && g.D <= 16) tall = 0;
+    const bool never = KIND == TDV_COST_NCC && R == 4 && !FILT && g.Dw == 16;
+    if (!never && tiles >= tall && band_bytes<KIND, R, HP, FILT, 8>(g) <= kThreeBlocks) return 8;
+    return KIND == TDV_COST_BT || band_bytes<KIND, R, HP, FILT, 4>(g) <= kTwoBlocks ? 4 : 2;
+}
 
 template <int R, int DW, bool FILT, int TY>
 cudaError_t launch_fastwta_ty(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
                               cudaStream_t st) {
     constexpr int P = 16;
-    using B = Band<TDV_COST_SSD, R, P / 2, TY>;
-    const int bytes = (FILT ? B::floats_filtered(g) : B::floats(g)) * 4;
+    const int bytes = band_bytes<TDV_COST_SSD, R, P / 2, FILT, TY>(g);
     auto k = fastwta_band_kernel<R, P, DW, FILT, TY>;
     static std::atomic<unsigned long long> opted{0};
     if (bytes > 48 * 1024) {
@@ -660,8 +707,9 @@ cudaError_t launch_fastwta_ty(const ImgArg& L, const ImgArg& Rim, const Geom& g,
 template <int R, int DW, bool FILT>
 cudaError_t launch_fastwta_dw(const ImgArg& L, const ImgArg& Rim, const Geom& g, uint16_t* disp, float* disp_norm,
                               cudaStream_t st) {
-    return tall_tiles(L.W, L.H) ? launch_fastwta_ty<R, DW, FILT, 8>(L, Rim, g, disp, disp_norm, st)
-                                : launch_fastwta_ty<R, DW, FILT, 4>(L, Rim, g, disp, disp_norm, st);
+    return tile_rows<TDV_COST_SSD, R, 8, FILT>(L.W, L.H, g) == 8
+               ? launch_fastwta_ty<R, DW, FILT, 8>(L, Rim, g, disp, disp_norm, st)
+               : launch_fastwta_ty<R, DW, FILT, 4>(L, Rim, g, disp, disp_norm, st);
 }
 
 template <int R, bool FILT>
@@ -672,12 +720,11 @@ cudaError_t launch_fastwta_r(const ImgArg& L, const ImgArg& Rim, const Geom& g, 
     return launch_fastwta_dw<R, 8, FILT>(L, Rim, g, disp, disp_norm, st);
 }
 
-template <int KIND, int R, int P, bool FILT, int TY>
-cudaError_t launch_ty(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
+template <int KIND, int R, int P, bool FILT, int TY, int NR>
+cudaError_t launch_nr(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
                       cudaStream_t st) {
-    using B = Band<KIND, R, P / 2, TY>;
-    const int bytes = (FILT ? B::floats_filtered(g) : B::floats(g)) * 4;
-    auto k = cost_band_kernel<KIND, R, P, FILT, TY>;
+    const int bytes = band_bytes<KIND, R, P / 2, FILT, TY>(g);
+    auto k = cost_band_kernel<KIND, R, P, FILT, TY, NR>;
     static std::atomic<unsigned long long> opted{0};
     if (bytes > 48 * 1024) {
         const cudaError_t e = opt_in_once(k, opted);
@@ -688,16 +735,42 @@ cudaError_t launch_ty(const ImgArg& L, const ImgArg& Rim, const VolArg& out, con
     return cudaGetLastError();
 }
 
+template <int KIND, int R, int P, bool FILT, int TY>
+cudaError_t launch_ty(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
+                      cudaStream_t st) {
+    // NCC of narrow lane groups: one row per item, so that every warp has one
+    // (9x9, 160x120, D = 16: 14 us, with two rows 19)
+    if constexpr (KIND == TDV_COST_NCC && TY > 2)
+        if (g.Dw < 32) return launch_nr<KIND, R, P, FILT, TY, 1>(L, Rim, out, g, fl_out, st);
+    return launch_nr<KIND, R, P, FILT, TY, 2>(L, Rim, out, g, fl_out, st);
+}
+
 template <int KIND, int R, int P, bool FILT>
 cudaError_t launch_one(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
                        cudaStream_t st) {
-    return tall_tiles(out.W, out.H) ? launch_ty<KIND, R, P, FILT, 8>(L, Rim, out, g, fl_out, st)
-                                    : launch_ty<KIND, R, P, FILT, 4>(L, Rim, out, g, fl_out, st);
+    switch (tile_rows<KIND, R, P / 2, FILT>(out.W, out.H, g)) {
+        case 8: return launch_ty<KIND, R, P, FILT, 8>(L, Rim, out, g, fl_out, st);
+        case 4: return launch_ty<KIND, R, P, FILT, 4>(L, Rim, out, g, fl_out, st);
+    }
+    if constexpr (KIND != TDV_COST_BT) return launch_ty<KIND, R, P, FILT, 2>(L, Rim, out, g, fl_out, st);
+    return cudaErrorInvalidValue;
 }
 
 template <int KIND, bool FILT>
 cudaError_t dispatch_r(int r, const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
                        cudaStream_t st) {
+    if constexpr (KIND == TDV_COST_NCC) {
+        // four pixel groups a warp: runs of 8 pixels, or the groups' pairs of
+        // right columns share banks (9x9, 640x480, D = 8: 35 us against 48)
+        if (g.Dw == 8) {
+            switch (r) {
+                case 1: return launch_one<KIND, 1, 8, FILT>(L, Rim, out, g, fl_out, st);
+                case 2: return launch_one<KIND, 2, 8, FILT>(L, Rim, out, g, fl_out, st);
+                case 3: return launch_one<KIND, 3, 8, FILT>(L, Rim, out, g, fl_out, st);
+                default: return launch_one<KIND, 4, 8, FILT>(L, Rim, out, g, fl_out, st);
+            }
+        }
+    }
     switch (r) {
         case 1: return launch_one<KIND, 1, 16, FILT>(L, Rim, out, g, fl_out, st);
         case 2: return launch_one<KIND, 2, 16, FILT>(L, Rim, out, g, fl_out, st);
@@ -708,7 +781,7 @@ cudaError_t dispatch_r(int r, const ImgArg& L, const ImgArg& Rim, const VolArg& 
 
 template <int KIND, int R>
 long long band_floats_r(const Geom& g, bool filt) {
-    using B = Band<KIND, R, KIND == TDV_COST_BT ? 4 : 8, 8>;  // the taller tile's
+    using B = Band<KIND, R, KIND == TDV_COST_BT ? 4 : 8, 4>;  // the lower tile's
     return filt ? B::floats_filtered(g) : B::floats(g);
 }
 

@@ -26,7 +26,7 @@
 // loads run ahead in a register ring.  The runs of L are padded to a multiple
 // of 8 disparities, so L always does: eight 4-byte stores per lane at a stride
 // of 32 bytes instead took D = 127 at 1920x1080 from 6.3 ms in sequence to 7.9,
-// and D = 60 at 3840x2160 from 11.0 to 17.8; padded they take 5.2 and 10.2.
+// and D = 60 at 3840x2160 from 11.0 to 17.8; padded they take 4.3 and 10.2.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 

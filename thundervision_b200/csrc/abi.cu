@@ -1012,6 +1012,7 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         TDV_TRY(ensure_side(ctx));
     }
     if (fused && tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
+        tdv::dirs_pays(W, H, D, params->paths, fp.excl, out->lr_threshold >= 0 || out->disp_right) &&
         dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, capturing(S(stream)))) {
         TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);

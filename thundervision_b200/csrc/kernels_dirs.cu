@@ -1221,6 +1221,16 @@ bool dirs_supported(int W, int H, int D, int p1h, int p2h, int excl) {
     return true;
 }
 
+// Long strips over four paths with D = 64 and the left-right check keep the
+// accumulating passes: their rows are the call's time (no vertical line is long
+// enough to matter), and where D fills a warp's span one line a warp steps
+// faster than four.  Accumulating / this, us: CPU recurrence 4096x300 1089 /
+// 1130, 16384x64 3220 / 3852 (4096x400 1181 / 1172, 2048x128 497 / 440); the
+// others 12288x64 2098 / 2210, 16384x64 2787 / 2978 (8192x64 1411 / 1364).
+bool dirs_pays(int W, int H, int D, int paths, int excl, int lr) {
+    return !(paths == 4 && D == 64 && lr && W > 12 * H && W >= (excl ? 4096 : 12288));
+}
+
 // Offset of the CPU recurrence: at least 510 + max(P1, P2 - P1), a multiple of 256.
 static int dirs_offset(int p1h, int p2h, int excl) {
     return excl ? (510 + std::max(p1h, p2h - p1h) + 255) / 256 * 256 : 0;

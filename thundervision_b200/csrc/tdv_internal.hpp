@@ -341,6 +341,7 @@ cudaError_t launch_fused(const FusedArgs& a, cudaStream_t st, Timer* tm);
 // of dirs_bytes(); agg2, the side stream and events, off_h and side are not
 // used.
 bool dirs_supported(int W, int H, int D, int p1h, int p2h, int excl);
+bool dirs_pays(int W, int H, int D, int paths, int excl, int lr);
 size_t dirs_plane_bytes(int W, int H);
 size_t dirs_bytes(int W, int H, int D, int paths, int excl);
 cudaError_t launch_dirs(const FusedArgs& a, cudaStream_t st, Timer* tm);

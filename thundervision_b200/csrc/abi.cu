@@ -118,6 +118,21 @@ bool grow_optional(tdv_ctx* ctx, tdv_ctx::OptBuf& b, size_t bytes) {
     return true;
 }
 
+// Whether an event recorded outside any capture has passed, asked while a
+// stream of this thread may be capturing.
+bool idle(cudaEvent_t ev) {
+    if (!ev) return true;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const bool done = cudaEventQuery(ev) == cudaSuccess;
+    if (!done) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return done;
+}
+
 // Scratch of the directions stored apart, where the allocator has room for it
 // (or an earlier call had, if the stream is capturing): false sends the call
 // to the accumulating passes, which need a quarter to a half of it.  It is
@@ -234,26 +249,49 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
 // the allocator has no room for them (the passes then run in sequence on S), and
 // where groups of four do not pay: under the CPU recurrence up to D = 64 their
 // sum, with its table of line counts, takes what the walks gain (3840x2160,
-// D = 60: 12.98 ms against 12.18 in sequence).  A capturing call takes what is
-// there.
-int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool captured) {
+// D = 60: 12.98 ms against 12.18 in sequence).
+//
+// Direct calls share sgm_part: each waits for the one before it, on whatever
+// stream that ran.  A capturing call allocates nothing and its replays run
+// beside direct calls, so it takes sgm_part over for good (idle, and larger than
+// what earlier captures took) as sgm_graph, and the next direct call allocates
+// again.  Replays that share sgm_graph also share the context's aggregation
+// volume; a capture into the caller's own volume shares nothing with any other
+// call, and stays so: in sequence.
+int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool own, cudaStream_t st, tdv_ctx::OptBuf** part) {
     const size_t vol = tdv::sgm_dirs_volume(W, H, D);
     const int np = (int)ctx->sched.passes.size();
     const int all = std::min(np, tdv::kMaxSideBySide);
     const bool fit = all * vol <= (size_t)10000000000;
     if (!fit && sem == TDV_SEM_REF_CPU && D <= 64) return 0;
-    for (int g : {fit ? all : std::min(all, 4), std::min(all, 2)}) {
-        const size_t need = g * vol;
-        if (ctx->sgm_part.bytes >= need) {
-            if ((uintptr_t)ctx->sgm_part.ptr & 31) return 0;
-            ctx->sgm_part.pinned = ctx->sgm_part.pinned || captured;
-            return g;
+    const bool captured = capturing(st);
+    if (captured && own) return 0;
+    const int most = fit ? all : std::min(all, 4);
+    if (captured && ctx->sgm_graph.bytes < most * vol && ctx->sgm_part.bytes > ctx->sgm_graph.bytes &&
+        ctx->retired_bytes + ctx->sgm_graph.bytes <= kMaxRetired && idle(ctx->sgm_done)) {
+        if (ctx->sgm_graph.ptr) {
+            ctx->retired.push_back(ctx->sgm_graph);
+            ctx->retired_bytes += ctx->sgm_graph.bytes;
         }
-        if (captured || need >= ctx->sgm_part_refused) continue;
-        if (grow_optional(ctx, ctx->sgm_part, need)) return ((uintptr_t)ctx->sgm_part.ptr & 31) ? 0 : g;
-        ctx->sgm_part_refused = need;
+        ctx->sgm_graph = ctx->sgm_part;
+        ctx->sgm_part = tdv_ctx::OptBuf();
     }
-    return 0;
+    tdv_ctx::OptBuf& b = captured ? ctx->sgm_graph : ctx->sgm_part;
+    *part = &b;
+    int group = 0;
+    for (int g : {most, std::min(all, 2)}) {
+        const size_t need = g * vol;
+        if (b.bytes < need) {
+            if (captured || need >= ctx->sgm_part_refused) continue;
+            if (!grow_optional(ctx, b, need)) {
+                ctx->sgm_part_refused = need;
+                continue;
+            }
+        }
+        group = g;
+        break;
+    }
+    return ((uintptr_t)b.ptr & 31) ? 0 : group;
 }
 
 tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
@@ -272,7 +310,11 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     a.p2_adjust = p->p2_mode == TDV_P2_ADJUST;
     a.sem = p->semantics;
     const bool lr = out->lr_threshold >= 0 || out->disp_right;
-    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, p->semantics, capturing(st)) : 0;
+    // the sequential passes' scratch whether or not they run: a later captured call may
+    if (ctx->sched.defer_rows > 0)
+        TDV_TRY(ensure(ctx, ctx->defer, (size_t)ctx->sched.defer_rows * D * sizeof(float)));
+    tdv_ctx::OptBuf* part = nullptr;
+    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, p->semantics, aggreg != nullptr, st, &part) : 0;
     const bool keep = aggreg || lr;  // the aggregated volume itself is needed
     VolArg Sv;
     if (aggreg) {
@@ -292,11 +334,16 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
         disp = (uint16_t*)ctx->misc.ptr;
     }
     if (group) {
-        TDV_CUDA(tdv::launch_sgm_dirs(a, ctx->sched, (float*)ctx->sgm_part.ptr, group, (float*)Sv.ptr, keep, disp,
-                                      out->disp_norm, st, &ctx->timer));
+        const bool direct = part == &ctx->sgm_part;
+        if (direct) {
+            if (ctx->sgm_done) TDV_CUDA(cudaStreamWaitEvent(st, ctx->sgm_done, 0));
+            else TDV_CUDA(cudaEventCreateWithFlags(&ctx->sgm_done, cudaEventDisableTiming));
+        }
+        const cudaError_t e = tdv::launch_sgm_dirs(a, ctx->sched, (float*)part->ptr, group, (float*)Sv.ptr, keep, disp,
+                                                   out->disp_norm, st, &ctx->timer);
+        if (direct) TDV_CUDA(cudaEventRecord(ctx->sgm_done, st));
+        TDV_CUDA(e);
     } else {
-        if (ctx->sched.defer_rows > 0)
-            TDV_TRY(ensure(ctx, ctx->defer, (size_t)ctx->sched.defer_rows * D * sizeof(float)));
         a.defer = ctx->sched.defer_rows > 0 ? (float*)ctx->defer.ptr : nullptr;
         TDV_CUDA(tdv::launch_sgm_passes(a, ctx->sched, st, &ctx->timer));
         TDV_CUDA(tdv::launch_wta(Sv, disp, out->disp_norm, st, &ctx->timer));
@@ -574,7 +621,8 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
                      ctx->misc.ptr || ctx->sched_buf.ptr || ctx->err.ptr || ctx->soft.ptr ||
                      ctx->agg2.ptr || ctx->defer.ptr || ctx->side || ctx->fw_buf.ptr || ctx->fside.ptr ||
                      ctx->lane_main || ctx->planes_b.ptr || ctx->agg_b.ptr || ctx->agg2_b.ptr || ctx->fside_b.ptr ||
-                     ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr || !ctx->retired.empty();
+                     ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr || ctx->sgm_graph.ptr || ctx->sgm_done ||
+                     !ctx->retired.empty();
     if (any) {
         DeviceScope ds(ctx->device);
         cudaDeviceSynchronize();
@@ -600,6 +648,8 @@ void tdv_ctx_destroy(tdv_ctx* ctx) {
         release_buf(ctx, ctx->dirs);
         release_buf(ctx, ctx->dirs_b);
         release_buf(ctx, ctx->sgm_part);
+        release_buf(ctx, ctx->sgm_graph);
+        if (ctx->sgm_done) cudaEventDestroy(ctx->sgm_done);
         for (tdv_ctx::Buf& b : ctx->retired) release_buf(ctx, b);
         if (ctx->lane_main) cudaStreamDestroy(ctx->lane_main);
         if (ctx->lane_side) cudaStreamDestroy(ctx->lane_side);
@@ -618,7 +668,8 @@ tdv_status tdv_ctx_set_allocator(tdv_ctx* ctx, tdv_alloc_fn alloc, tdv_free_fn r
     if ((alloc == nullptr) != (release == nullptr))
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator and release must be set together");
     if (ctx->agg.ptr || ctx->cost.ptr || ctx->planes.ptr || ctx->codes.ptr || ctx->misc.ptr ||
-        ctx->sched_buf.ptr || ctx->defer.ptr || ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr)
+        ctx->sched_buf.ptr || ctx->defer.ptr || ctx->dirs.ptr || ctx->dirs_b.ptr || ctx->sgm_part.ptr ||
+        ctx->sgm_graph.ptr)
         return fail(ctx, TDV_ERR_INVALID_ARG, "allocator must be set before any scratch exists");
     ctx->alloc = alloc;
     ctx->release = release;

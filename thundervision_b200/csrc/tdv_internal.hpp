@@ -206,8 +206,12 @@ struct tdv_ctx {
     OptBuf dirs, dirs_b;
     size_t dirs_refused = (size_t)-1;
     // general path with the passes side by side (kernels_sgm_dirs.cu)
-    OptBuf sgm_part;
+    // -- direct calls' volumes with the event after their last use, on which a
+    // call on any stream waits, and the volumes captured calls write (no direct
+    // call does: a replay may run beside it)
+    OptBuf sgm_part, sgm_graph;
     size_t sgm_part_refused = (size_t)-1;
+    cudaEvent_t sgm_done = nullptr;
     std::vector<Buf> retired;   // pinned buffers that were outgrown
     size_t retired_bytes = 0;
     cudaStream_t lane_main = nullptr, lane_side = nullptr;

@@ -94,15 +94,17 @@ bool capturing(cudaStream_t st) {
     return c != cudaStreamCaptureStatusNone;
 }
 
-// Outgrown buffers that graphs hold: at most this much per context.
-constexpr size_t kMaxRetired = (size_t)10000000000;
+// Scratch a call can do without takes at most this much per use: the volumes of
+// the directions stored apart (each lane), the general path's passes side by
+// side, and the outgrown buffers that graphs hold.
+constexpr size_t kMaxOptional = (size_t)10000000000;
 
 // Grows scratch a call can do without; a refusal leaves the buffer as it was.
 // The new buffer comes first, then the old one goes: set aside if a graph
 // holds its address, else freed once queued work is through with it.
 bool grow_optional(tdv_ctx* ctx, tdv_ctx::OptBuf& b, size_t bytes) {
     if (b.bytes >= bytes) return true;
-    if (b.pinned && ctx->retired_bytes + b.bytes > kMaxRetired) return false;
+    if (b.pinned && ctx->retired_bytes + b.bytes > kMaxOptional) return false;
     void* p = device_alloc(ctx, bytes);
     if (!p) return false;
     if (b.pinned) {
@@ -138,14 +140,18 @@ bool idle(cudaEvent_t ev) {
 // to the accumulating passes, which need a quarter to a half of it.  It is
 // sized like the accumulation volumes, by W x H and the class of D alone (8
 // paths, the CPU recurrence's words), so that it grows only where they do; by
-// this call's own need where that is refused.
+// this call's own need where that is refused or above kMaxOptional.  Calls
+// within a reserved size take what the reservation left.
 bool dirs_ready(tdv_ctx* ctx, tdv_ctx::OptBuf& b, int W, int H, int D, int paths, int excl, bool captured) {
     const size_t need = tdv::dirs_bytes(W, H, D, paths, excl);
     if (b.bytes < need) {
-        if (captured || need >= ctx->dirs_refused) return false;
+        if (captured || need > kMaxOptional || need >= ctx->dirs_refused) return false;
+        if (&b == &ctx->dirs)
+            for (const tdv_ctx::Extent& r : ctx->reserved)
+                if (W <= r.W && H <= r.H && D <= r.D) return false;
         const int dclass = (int)(tdv::fused_agg_bytes(1, 1, D) / sizeof(uint16_t));
         const size_t all = tdv::dirs_bytes(W, H, dclass, 8, 1);
-        if ((all >= ctx->dirs_refused || !grow_optional(ctx, b, all)) &&
+        if ((all > kMaxOptional || all >= ctx->dirs_refused || !grow_optional(ctx, b, all)) &&
             (all == need || !grow_optional(ctx, b, need))) {
             ctx->dirs_refused = need;
             return false;
@@ -262,13 +268,13 @@ int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool own, cudaStrea
     const size_t vol = tdv::sgm_dirs_volume(W, H, D);
     const int np = (int)ctx->sched.passes.size();
     const int all = std::min(np, tdv::kMaxSideBySide);
-    const bool fit = all * vol <= (size_t)10000000000;
+    const bool fit = all * vol <= kMaxOptional;
     if (!fit && sem == TDV_SEM_REF_CPU && D <= 64) return 0;
     const bool captured = capturing(st);
     if (captured && own) return 0;
     const int most = fit ? all : std::min(all, 4);
     if (captured && ctx->sgm_graph.bytes < most * vol && ctx->sgm_part.bytes > ctx->sgm_graph.bytes &&
-        ctx->retired_bytes + ctx->sgm_graph.bytes <= kMaxRetired && idle(ctx->sgm_done)) {
+        ctx->retired_bytes + ctx->sgm_graph.bytes <= kMaxOptional && idle(ctx->sgm_done)) {
         if (ctx->sgm_graph.ptr) {
             ctx->retired.push_back(ctx->sgm_graph);
             ctx->retired_bytes += ctx->sgm_graph.bytes;
@@ -683,7 +689,16 @@ tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t W, int32_t H, int32_t D) {
         return fail(ctx, TDV_ERR_INVALID_ARG, "bad reserve size %dx%dx%d", W, H, D);
     auto reserve = [&]() -> tdv_status {
         TDV_TRY(reserve_fused(ctx, W, H, D));
-        if (D <= tdv::kMaxDispSgm) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, false);
+        if (D > tdv::kMaxDispSgm) return TDV_OK;
+        // every direction's volume where a call of this size may use them;
+        // their refusal is not an error
+        std::vector<tdv_ctx::Extent> others;
+        for (const tdv_ctx::Extent& r : ctx->reserved)
+            if (r.W > W || r.H > H || r.D > D) others.push_back(r);
+        ctx->reserved.clear();
+        if (tdv::dirs_supported(W, H, D, 0, 0, 0)) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, false);
+        others.push_back({W, H, D});
+        ctx->reserved = std::move(others);
         return TDV_OK;
     };
     if (!ctx->alloc) {

@@ -203,7 +203,12 @@ struct tdv_ctx {
     // fused path with the directions stored apart (kernels_dirs.cu), per lane;
     // dirs_refused: the smallest such request the allocator turned down, so
     // that later calls of that size go straight to the accumulating passes
+    // reserved: the sizes tdv_ctx_reserve was given, within which no call grows `dirs`
     OptBuf dirs, dirs_b;
+    struct Extent {
+        int W, H, D;
+    };
+    std::vector<Extent> reserved;
     size_t dirs_refused = (size_t)-1;
     // general path with the passes side by side (kernels_sgm_dirs.cu)
     // -- direct calls' volumes with the event after their last use, on which a

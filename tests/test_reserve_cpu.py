@@ -70,6 +70,16 @@ def test_no_volumes_no_call_can_use(make, W, H, D):
     assert len(asked) == 4 and max(asked) == W * H * D * 2
 
 
+def test_reserving_again_after_a_refusal(make):
+    c = make(limit=1 << 30)
+    assert len(c.reserve(1024, 768, 256)) >= 5 and len(c.live) == 4
+    c.limit = 1 << 60
+    c.reserve(1024, 768, 256)
+    assert len(c.live) == 5
+    # the refusal was no error of the call that met it
+    assert c.lib.tdv_last_error_string(c.h) == b""
+
+
 def test_smaller_reservation_keeps_what_is_there(make):
     c = make()
     c.reserve(800, 600, 128)

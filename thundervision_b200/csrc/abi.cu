@@ -135,6 +135,16 @@ bool idle(cudaEvent_t ev) {
     return done;
 }
 
+// Whether to do without asking for `need` bytes: a refusal stands for 64 calls
+// (a refused request makes a caching allocator flush its cache), not for the
+// context's life: memory that was short once may be there again.
+bool refused(tdv_ctx::Refusal& r, size_t need) {
+    if (need < r.bytes) return false;
+    if (--r.calls > 0) return true;
+    r = tdv_ctx::Refusal();
+    return false;
+}
+
 // Scratch of the directions stored apart, where the allocator has room for it
 // (or an earlier call had, if the stream is capturing): false sends the call
 // to the accumulating passes, which need a quarter to a half of it.  It is
@@ -145,15 +155,16 @@ bool idle(cudaEvent_t ev) {
 bool dirs_ready(tdv_ctx* ctx, tdv_ctx::OptBuf& b, int W, int H, int D, int paths, int excl, bool captured) {
     const size_t need = tdv::dirs_bytes(W, H, D, paths, excl);
     if (b.bytes < need) {
-        if (captured || need > kMaxOptional || need >= ctx->dirs_refused) return false;
+        if (captured || need > kMaxOptional) return false;
         if (&b == &ctx->dirs)
             for (const tdv_ctx::Extent& r : ctx->reserved)
                 if (W <= r.W && H <= r.H && D <= r.D) return false;
+        if (refused(ctx->dirs_refused, need)) return false;
         const int dclass = (int)(tdv::fused_agg_bytes(1, 1, D) / sizeof(uint16_t));
         const size_t all = tdv::dirs_bytes(W, H, dclass, 8, 1);
-        if ((all > kMaxOptional || all >= ctx->dirs_refused || !grow_optional(ctx, b, all)) &&
+        if ((all > kMaxOptional || all >= ctx->dirs_refused.bytes || !grow_optional(ctx, b, all)) &&
             (all == need || !grow_optional(ctx, b, need))) {
-            ctx->dirs_refused = need;
+            ctx->dirs_refused = {need, 64};
             return false;
         }
     }
@@ -288,9 +299,9 @@ int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool own, cudaStrea
     for (int g : {most, std::min(all, 2)}) {
         const size_t need = g * vol;
         if (b.bytes < need) {
-            if (captured || need >= ctx->sgm_part_refused) continue;
+            if (captured || refused(ctx->sgm_refused, need)) continue;
             if (!grow_optional(ctx, b, need)) {
-                ctx->sgm_part_refused = need;
+                ctx->sgm_refused = {need, 64};
                 continue;
             }
         }
@@ -696,6 +707,7 @@ tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t W, int32_t H, int32_t D) {
         for (const tdv_ctx::Extent& r : ctx->reserved)
             if (r.W > W || r.H > H || r.D > D) others.push_back(r);
         ctx->reserved.clear();
+        ctx->dirs_refused = tdv_ctx::Refusal();
         if (tdv::dirs_supported(W, H, D, 0, 0, 0)) dirs_ready(ctx, ctx->dirs, W, H, D, 8, 1, false);
         others.push_back({W, H, D});
         ctx->reserved = std::move(others);

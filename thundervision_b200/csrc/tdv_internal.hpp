@@ -200,22 +200,26 @@ struct tdv_ctx {
     // lane's planes, volumes and side rows, its two streams, its chains'
     // fork/join events and the events that tie it to the call's stream
     Buf planes_b, agg_b, agg2_b, fside_b;
-    // fused path with the directions stored apart (kernels_dirs.cu), per lane;
-    // dirs_refused: the smallest such request the allocator turned down, so
-    // that later calls of that size go straight to the accumulating passes
+    // The smallest request for such scratch that the allocator turned down: the
+    // next calls of that size do without asking, until `calls` runs out.
+    struct Refusal {
+        size_t bytes = (size_t)-1;
+        int calls = 0;
+    };
+    // fused path with the directions stored apart (kernels_dirs.cu), per lane
     // reserved: the sizes tdv_ctx_reserve was given, within which no call grows `dirs`
     OptBuf dirs, dirs_b;
     struct Extent {
         int W, H, D;
     };
     std::vector<Extent> reserved;
-    size_t dirs_refused = (size_t)-1;
+    Refusal dirs_refused;
     // general path with the passes side by side (kernels_sgm_dirs.cu)
     // -- direct calls' volumes with the event after their last use, on which a
     // call on any stream waits, and the volumes captured calls write (no direct
     // call does: a replay may run beside it)
     OptBuf sgm_part, sgm_graph;
-    size_t sgm_part_refused = (size_t)-1;
+    Refusal sgm_refused;
     cudaEvent_t sgm_done = nullptr;
     std::vector<Buf> retired;   // pinned buffers that were outgrown
     size_t retired_bytes = 0;

@@ -21,6 +21,7 @@ namespace {
 
 using tdv_abi::DeviceScope;
 using tdv_abi::device_alloc;
+using tdv_abi::device_alloc_needed;
 using tdv_abi::device_free;
 using tdv_abi::ensure;
 using tdv_abi::fail;
@@ -330,8 +331,6 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     // the sequential passes' scratch whether or not they run: a later captured call may
     if (ctx->sched.defer_rows > 0)
         TDV_TRY(ensure(ctx, ctx->defer, (size_t)ctx->sched.defer_rows * D * sizeof(float)));
-    tdv_ctx::OptBuf* part = nullptr;
-    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, p->semantics, aggreg != nullptr, st, &part) : 0;
     const bool keep = aggreg || lr;  // the aggregated volume itself is needed
     VolArg Sv;
     if (aggreg) {
@@ -350,6 +349,9 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
         TDV_TRY(ensure(ctx, ctx->misc, (size_t)W * H * sizeof(uint16_t)));
         disp = (uint16_t*)ctx->misc.ptr;
     }
+    // last: an allocation after it could give these volumes back
+    tdv_ctx::OptBuf* part = nullptr;
+    const int group = ctx->sched.lines ? side_by_side(ctx, W, H, D, p->semantics, aggreg != nullptr, st, &part) : 0;
     if (group) {
         const bool direct = part == &ctx->sgm_part;
         if (direct) {
@@ -1088,11 +1090,11 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
     if (fused) {
         TDV_TRY(reserve_fused(ctx, W, H, D));
         TDV_TRY(ensure_side(ctx));
+        TDV_TRY(ensure_err(ctx, S(stream)));
     }
     if (fused && tdv::dirs_supported(W, H, D, fp.p1h, fp.p2h, fp.excl) &&
         tdv::dirs_pays(W, H, D, params->paths, fp.excl, out->lr_threshold >= 0 || out->disp_right) &&
         dirs_ready(ctx, ctx->dirs, W, H, D, params->paths, fp.excl, capturing(S(stream)))) {
-        TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
         a.planes = ctx->planes.ptr;
         a.agg = ctx->dirs.ptr;
@@ -1100,7 +1102,6 @@ tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* 
         return TDV_OK;
     }
     if (fused) {
-        TDV_TRY(ensure_err(ctx, S(stream)));
         tdv::FusedArgs a = fused_args(ctx, left, right, D, params, fp, out);
         a.planes = ctx->planes.ptr;
         a.agg = ctx->agg.ptr;
@@ -1240,7 +1241,7 @@ tdv_status batch_replan(tdv_batch* b, const tdv_batch_tiles& t) {
         if (plan.bytes > b->desc_bytes) {
             // the descriptors hold the queue's own address: grow, then plan again
             device_free(ctx, b->desc);
-            b->desc = device_alloc(ctx, plan.bytes);
+            b->desc = device_alloc_needed(ctx, plan.bytes);
             b->desc_bytes = b->desc ? plan.bytes : 0;
             if (!b->desc) return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of work queue failed", plan.bytes);
             continue;
@@ -1323,7 +1324,7 @@ tdv_status tdv_batch_create(tdv_ctx* ctx, const tdv_batch_pair* pairs, int32_t n
     if (db) b->scratch = device_alloc(ctx, db);
     b->dirs = b->scratch != nullptr;
     const size_t sb = tdv::batch_scratch_bytes(b->pairs);
-    if (!b->dirs) b->scratch = device_alloc(ctx, sb);
+    if (!b->dirs) b->scratch = device_alloc_needed(ctx, sb);
     if (!b->scratch) {
         delete b;
         return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of batch scratch failed", sb);

@@ -61,6 +61,31 @@ inline void device_free(tdv_ctx* ctx, void* p) {
     else cudaFree(p);
 }
 
+// Gives the context's optional scratch back (what no graph holds), so that a
+// call's necessary scratch fits where it did before a context held any.
+inline bool give_back(tdv_ctx* ctx) {
+    tdv_ctx::OptBuf* const opt[] = {&ctx->dirs, &ctx->dirs_b, &ctx->sgm_part};
+    bool any = false;
+    for (const tdv_ctx::OptBuf* b : opt) any = any || (b->ptr && !b->pinned);
+    if (!any) return false;
+    if (cudaDeviceSynchronize() != cudaSuccess) {  // queued work may use it
+        cudaGetLastError();
+        return false;
+    }
+    for (tdv_ctx::OptBuf* b : opt)
+        if (!b->pinned) {
+            device_free(ctx, b->ptr);
+            *b = tdv_ctx::OptBuf();
+        }
+    return true;
+}
+
+// Necessary device memory: asked for once more after giving back.
+inline void* device_alloc_needed(tdv_ctx* ctx, size_t bytes) {
+    void* p = device_alloc(ctx, bytes);
+    return !p && give_back(ctx) ? device_alloc(ctx, bytes) : p;
+}
+
 // Scratch buffers grow on demand; growing waits for the device first because
 // work already queued may still read the old buffer.
 inline tdv_status ensure(tdv_ctx* ctx, tdv_ctx::Buf& b, size_t bytes) {
@@ -72,7 +97,7 @@ inline tdv_status ensure(tdv_ctx* ctx, tdv_ctx::Buf& b, size_t bytes) {
         b.ptr = nullptr;
         b.bytes = 0;
     }
-    void* p = device_alloc(ctx, bytes);
+    void* p = device_alloc_needed(ctx, bytes);
     if (!p) return fail(ctx, TDV_ERR_OOM, "allocating %zu bytes of scratch failed", bytes);
     b.ptr = p;
     b.bytes = bytes;

@@ -374,7 +374,7 @@ cudaError_t configure_nw(const BatchPlan& plan) {
     cudaError_t e = cudaFuncGetAttributes(&fa, batch_kernel<NW>);
     if (e != cudaSuccess) return e;
     if (fa.maxThreadsPerBlock < NW * 32) return cudaErrorInvalidConfiguration;
-    return cudaFuncSetAttribute(batch_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem);
+    return opt_in_smem((const void*)batch_kernel<NW>, plan.smem);
 }
 
 cudaError_t batch_configure(const BatchPlan& plan) {

@@ -53,7 +53,6 @@
 // recurrence adds P1 to a line's first costs before its second step (GS).
 // Which directions count in a pixel, and how often, is applied by the sum.
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -1132,15 +1131,8 @@ cudaError_t launch_dirs_pass(const EK& k, cudaStream_t st) {
     using C = Cfg<LPG, LNT>;
     int nh, nv, ng;
     const int blocks = line_blocks<C>(k.W, k.H, k.nd, nh, nv, ng);
-    static std::atomic<unsigned long long> opted{0};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    const cudaError_t e = opt_in_smem((const void*)dirs_pass_kernel<LPG, LNT, EXCL>, C::SMEM);
     if (e != cudaSuccess) return e;
-    if (dev >= 64 || !((opted.load() >> dev) & 1ull)) {
-        e = cudaFuncSetAttribute(dirs_pass_kernel<LPG, LNT, EXCL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-        if (e != cudaSuccess) return e;
-        if (dev < 64) opted.fetch_or(1ull << dev);
-    }
     dirs_pass_kernel<LPG, LNT, EXCL><<<blocks, C::T, C::SMEM, st>>>(k, nh, nv, ng);
     return cudaGetLastError();
 }
@@ -1169,7 +1161,7 @@ cudaError_t launch_dirs_sum(const EK& k, SumOut o, bool lr, cudaStream_t st) {
     const int blocks = (k.H + o.rows - 1) / o.rows;
     auto kern = lr ? dirs_sum_kernel<LPG, ND, WTD, EXCL, true> : dirs_sum_kernel<LPG, ND, WTD, EXCL, false>;
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = opt_in_smem((const void*)kern, smem);
         if (e != cudaSuccess) return e;
     }
     kern<<<blocks, threads, smem, st>>>(k, o);
@@ -1451,11 +1443,9 @@ namespace {
 
 template <int ND>
 cudaError_t configure_nd(const BatchPlan& plan) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(batch_dirs_kernel<ND, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, plan.smem);
+    const cudaError_t e = opt_in_smem((const void*)batch_dirs_kernel<ND, false>, plan.smem);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(batch_dirs_kernel<ND, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                plan.sum_smem);
+    return opt_in_smem((const void*)batch_dirs_kernel<ND, true>, plan.sum_smem);
 }
 
 template <int ND>

@@ -88,22 +88,6 @@ int sm_count() {
     return cache[dev];
 }
 
-// Opts a kernel into `bytes` of dynamic shared memory on the current device,
-// once: later launches needing no more skip the driver call.
-cudaError_t opt_in_smem(const void* fn, int bytes) {
-    static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> done;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    int& cur = done[{fn, dev}];
-    if (bytes <= cur) return cudaSuccess;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) cur = bytes;
-    return e;
-}
-
 // Greedy pairing: groups by decreasing row count, each block takes the
 // longest left and, if it fits under the longest, the shortest left.
 // Returns the block count, or -1 if the table would overflow.
@@ -294,6 +278,20 @@ cudaError_t run_fused(const FK& k, const FusedArgs& a, cudaStream_t st, Timer* t
 }
 
 }  // namespace
+
+cudaError_t opt_in_smem(const void* fn, int bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, int> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    int& cur = done[{fn, dev}];
+    if (bytes <= cur) return cudaSuccess;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) cur = bytes;
+    return e;
+}
 
 size_t fused_plane_bytes(int W, int H) {
     return ((size_t)W * H + (size_t)padded_len(W) * H) * sizeof(Plane);

@@ -346,6 +346,11 @@ cudaError_t launch_subpixel(const float* S, int W, int H, int D, const uint16_t*
                             cudaStream_t st);
 cudaError_t launch_reproject(const RasterArg& disp, const RasterArg* color, int mode, float zscale,
                              const float* q, float* verts, float* cols, cudaStream_t st);
+// Opts a kernel into `bytes` of dynamic shared memory on the current device,
+// once: the limit is process-wide and is only ever raised, so a launch on
+// another thread that needs more keeps it, and later launches that need no more
+// skip the driver call.
+cudaError_t opt_in_smem(const void* fn, int bytes);
 size_t fused_plane_bytes(int W, int H);
 cudaError_t launch_fused(const FusedArgs& a, cudaStream_t st, Timer* tm);
 

@@ -253,7 +253,8 @@ tdv_status tdv_batch_set_tiles(tdv_batch* batch, const tdv_batch_tiles* tiles);
 tdv_status tdv_batch_get_tiles(const tdv_batch* batch, tdv_batch_tiles* tiles);
 /* Times candidate tile shapes on this batch (each run `reps` times on
  * `stream`, device time by CUDA events), keeps the fastest and returns it
- * with its milliseconds per run. */
+ * with its milliseconds per run.  Where the directions are stored apart only
+ * the two queue orders are candidates, and the other fields stay as set. */
 tdv_status tdv_batch_autotune(tdv_batch* batch, int32_t reps, tdv_stream stream,
                               tdv_batch_tiles* chosen, double* best_ms);
 /* One run: zero the queue's control words, then one persistent launch, or one

@@ -472,7 +472,8 @@ class Batch:
         self.ctx.check(L.lib().tdv_batch_set_tiles(self.handle, ctypes.byref(t)))
 
     def autotune(self, reps=3):
-        """Time candidate tile shapes, keep the fastest; returns (tiles, ms)."""
+        """Time candidate tile shapes, keep the fastest; returns (tiles, ms).
+        Batches that store the directions apart take only the queue order."""
         t = L.tdv_batch_tiles()
         ms = ctypes.c_double()
         self.ctx.check(L.lib().tdv_batch_autotune(self.handle, reps, _stream(), ctypes.byref(t),

@@ -1491,11 +1491,22 @@ tdv_status tdv_batch_autotune(tdv_batch* b, int32_t reps, tdv_stream stream, tdv
         wmax = std::max(wmax, p.W);
         hmax = std::max(hmax, p.H);
     }
+    if (b->dirs) {
+        // directions stored apart: the plan takes the queue order alone
+        tdv_batch_tiles t = best;
+        t.order = best.order == TDV_BATCH_ORDER_INPUT ? TDV_BATCH_ORDER_LONGEST_FIRST : TDV_BATCH_ORDER_INPUT;
+        double ms = HUGE_VAL;
+        if (st_all == TDV_OK) st_all = time_tiles(t, ms);
+        if (ms < best_t) {
+            best_t = ms;
+            best = t;
+        }
+    }
     // one coordinate descent per blocks-per-SM setting (it bounds the lines
     // and rows a block can take), over lines, rows, split and queue order;
     // besides fixed sizes, the sizes that give the largest pair one tile per
     // block slot
-    for (int ctas = 1; ctas <= 2 && st_all == TDV_OK; ctas++) {
+    for (int ctas = 1; !b->dirs && ctas <= 2 && st_all == TDV_OK; ctas++) {
         tdv_batch_tiles cur = b->tiles;
         cur.ctas_per_sm = ctas;
         double cur_t;

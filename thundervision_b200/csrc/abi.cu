@@ -355,8 +355,11 @@ tdv_status run_sgm(tdv_ctx* ctx, const tdv_volume* cost, const tdv_image* guide,
     if (group) {
         const bool direct = part == &ctx->sgm_part;
         if (direct) {
-            if (ctx->sgm_done) TDV_CUDA(cudaStreamWaitEvent(st, ctx->sgm_done, 0));
-            else TDV_CUDA(cudaEventCreateWithFlags(&ctx->sgm_done, cudaEventDisableTiming));
+            unsigned long long id = 0;
+            TDV_CUDA(cudaStreamGetId(st, &id));
+            if (!ctx->sgm_done) TDV_CUDA(cudaEventCreateWithFlags(&ctx->sgm_done, cudaEventDisableTiming));
+            else if (id != ctx->sgm_stream) TDV_CUDA(cudaStreamWaitEvent(st, ctx->sgm_done, 0));
+            ctx->sgm_stream = id;
         }
         const cudaError_t e = tdv::launch_sgm_dirs(a, ctx->sched, (float*)part->ptr, group, (float*)Sv.ptr, keep, disp,
                                                    out->disp_norm, st, &ctx->timer);

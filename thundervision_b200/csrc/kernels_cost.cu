@@ -46,7 +46,7 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxBandBytes = 220 * 1024;
 // columns the fused Gaussian of the window costs filters at a time
-constexpr int kFilterCols = 144;
+constexpr int kFilterCols = 208;
 constexpr int kThreeBlocks = 75 * 1024, kTwoBlocks = 113 * 1024;  // shared memory of a block, so many to an SM
 
 __device__ __forceinline__ float fetch(const ImgArg& im, int x, int y) {
@@ -332,10 +332,11 @@ __device__ void stage(const ImgArg& L, const ImgArg& Rim, const Geom& g, int x0,
         float* lb = sm;
         float* rb = sm + B::rband(g);
         float* scr = sm + B::scratch(g);
-        gauss_band<true>(L, x0 - R, kTX + 2 * R, y0 - R, B::kRows,
+        gauss_band<false>(L, x0 - R, kTX + 2 * R, y0 - R, B::kRows,
                    [&](int r, int c, float v) { B::put_left(lb + r * B::kLeft, c, v); }, scr);
-        gauss_band<true>(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows,
-                   [&](int r, int c, float v) { B::put_right(rb + r * g.rbw * 2, c, v); }, scr);
+        auto put = [&](int r, int c, float v) { B::put_right(rb + r * g.rbw * 2, c, v); };
+        if (g.rbw <= kFilterCols) gauss_band<false>(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows, put, scr);
+        else gauss_band<true>(Rim, x0 - (g.D - 1) - R, g.rbw, y0 - R, B::kRows, put, scr);
         if (fl_out)
             for (int i = tid; i < kTX * B::TY; i += kThreads) {
                 const int row = i / kTX, col = i - row * kTX;

@@ -151,10 +151,13 @@ __global__ void __launch_bounds__(128) sgm_dirs_kernel(SgmArgs a, const Walk* __
     const long long off = wk.sx * a.C.sx + wk.sy * a.C.sy + d0, stride = dx * a.C.sx + dy * a.C.sy;
     const CT* cq = (const CT*)a.C.ptr + off;
     // the path costs' runs are padded to whole lanes: always one 32-byte store
-    const int Dp = (D + 7) & ~7;
-    const long long px = a.C.sx / D, py = a.C.sy / D;  // pixels
-    float* lq = part + pi * vol + (wk.sx * px + wk.sy * py) * Dp + d0;
-    const long long lstride = (dx * px + dy * py) * Dp;
+    // (VEC: no padding, the costs' own offsets; they cost a 640x480, D = 128
+    // volume 6 % otherwise)
+    const int pad = VEC ? 0 : ((D + 7) & ~7) - D;
+    const bool xmajor = a.C.sx > a.C.sy;
+    const long long px = xmajor ? a.C.H : 1, py = xmajor ? 1 : a.C.W;  // pixels between neighbours
+    float* lq = part + pi * vol + off + (VEC ? 0 : (wk.sx * px + wk.sy * py) * pad);
+    const long long lstride = stride + (VEC ? 0 : (dx * px + dy * py) * pad);
     const int len = wk.len;
     const int steps = __reduce_max_sync(FULLM, len);
     constexpr int K = 4;  // steps of C in flight (two: 0.275 ms against 0.220 at 640x480, D = 64)
@@ -242,26 +245,28 @@ __global__ void __launch_bounds__(128) sgm_dirs_kernel(SgmArgs a, const Walk* __
 // the winner (strict '<' in increasing d: the lowest d wins a tie, NaN and
 // +INF never win, no finite value -> d = 0).  A warp per pixel, lane l holding
 // d = l, l + 32, ...: every load of the pixel is in flight before the first
-// addition.  PLAIN: every pass takes every cell once (no table look-ups).
+// addition.  PLAIN: every pass takes every cell once (no table look-ups).  PAD:
+// the volumes' runs are padded (as a run-time stride it cost 3 % where they are
+// not).
 struct SumArgs {
     const float* part;
     size_t vol;
     const float* Sin;        // S of the groups before this one, or null
     float* S;                // S stored, or null
     const uint16_t* mult;    // per pass nl line counts (0: no walk, n: n times)
-    int nl, W, H, D, Dp, xmajor;
+    int nl, W, H, D, xmajor;
     int dx[kMaxSideBySide], dy[kMaxSideBySide];
     int first;               // the group's first pass writes S
     uint16_t* disp;          // winners, or null
     float* disp_norm;
     int winner;
 };
-template <int N, int NP, bool PLAIN, bool REFCPU>
+template <int N, int NP, bool PLAIN, bool REFCPU, bool PAD>
 __global__ void __launch_bounds__(256) sgm_sum_kernel(SumArgs a) {
     const int lane = threadIdx.x & 31;
     const uint32_t npix = (uint32_t)a.W * (uint32_t)a.H, side = a.xmajor ? a.H : a.W;
     for (uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < npix; q += (gridDim.x * blockDim.x) >> 5) {
-        const float* p = a.part + (size_t)q * a.Dp + lane;
+        const float* p = a.part + (size_t)q * (PAD ? (a.D + 7) & ~7 : a.D) + lane;
         float v[N][NP], s[N];
 #pragma unroll
         for (int i = 0; i < N; i++)
@@ -365,12 +370,18 @@ cudaError_t run_group_any(const SgmArgs& a, const PassSchedule& sch, const DirGr
     }
 }
 
+template <int N, int NP, bool PAD>
+cudaError_t run_sum_pad(const SumArgs& s, bool plain, bool refcpu, int grid, cudaStream_t st) {
+    if (plain && !refcpu) sgm_sum_kernel<N, NP, true, false, PAD><<<grid, 256, 0, st>>>(s);
+    else if (!refcpu) sgm_sum_kernel<N, NP, false, false, PAD><<<grid, 256, 0, st>>>(s);
+    else sgm_sum_kernel<N, NP, false, true, PAD><<<grid, 256, 0, st>>>(s);
+    return cudaGetLastError();
+}
+
 template <int N, int NP>
 cudaError_t run_sum(const SumArgs& s, bool plain, bool refcpu, int grid, cudaStream_t st) {
-    if (plain && !refcpu) sgm_sum_kernel<N, NP, true, false><<<grid, 256, 0, st>>>(s);
-    else if (!refcpu) sgm_sum_kernel<N, NP, false, false><<<grid, 256, 0, st>>>(s);
-    else sgm_sum_kernel<N, NP, false, true><<<grid, 256, 0, st>>>(s);
-    return cudaGetLastError();
+    return s.D % 8 == 0 ? run_sum_pad<N, NP, false>(s, plain, refcpu, grid, st)
+                        : run_sum_pad<N, NP, true>(s, plain, refcpu, grid, st);
 }
 
 template <int N>
@@ -429,7 +440,6 @@ cudaError_t launch_sgm_dirs(const SgmArgs& a, const PassSchedule& sch, float* pa
         s.W = W;
         s.H = H;
         s.D = D;
-        s.Dp = (D + 7) & ~7;
         s.xmajor = a.C.sx > a.C.sy ? 1 : 0;
         s.first = g0 == 0;
         s.disp = disp;

@@ -216,11 +216,13 @@ struct tdv_ctx {
     Refusal dirs_refused;
     // general path with the passes side by side (kernels_sgm_dirs.cu)
     // -- direct calls' volumes with the event after their last use, on which a
-    // call on any stream waits, and the volumes captured calls write (no direct
+    // call on another stream (by its id, which no later stream takes over)
+    // waits, and the volumes captured calls write (no direct
     // call does: a replay may run beside it)
     OptBuf sgm_part, sgm_graph;
     Refusal sgm_refused;
     cudaEvent_t sgm_done = nullptr;
+    unsigned long long sgm_stream = 0;
     std::vector<Buf> retired;   // pinned buffers that were outgrown
     size_t retired_bytes = 0;
     cudaStream_t lane_main = nullptr, lane_side = nullptr;

@@ -445,7 +445,7 @@ def batch_trace_summary(tr, shapes):
 def measure_batch(ctx, dev, reps=3):
     """Uneven batch: 64 seeded pairs, W ~ U[320,1920], H ~ U[240,1080] (multiples
     of 16), D in {32,64,128,256}; BT + SGM-8 + WTA.  One graph-captured
-    persistent launch with autotuned tiles vs (a) 64 per-pair launches of the
+    batch run with the queue order autotuned vs (a) 64 per-pair launches of the
     plain method -- BT cost DSI (tdv_cost, FP32) then SGM + WTA (tdv_sgm) --
     and (b) 64 per-pair launches of the fused path (tdv_stereo_sgm); outputs
     and the DSI preallocated, all on one stream, device time."""
@@ -819,10 +819,11 @@ def measure_video(ctx, dev, n_frames=300, refit_steps=50):
     """Full-HD video: 300 frames (12 moving rectangles over a slanted plane,
     sensor noise sigma 2), D=256, fused BT + SGM + WTA + L-R check, through a
     double-buffered loop of per-frame graph replays (the fused kernels, and
-    beside them the persistent batch kernel) with every frame copied from
-    pinned host memory and its map copied back (timed), 4-path vs 8-path; then P1/P2 fitted by 50 Adam steps on the soft-argmin L1
-    loss (FP32 BT volume, adjoint kernels) and the refit vs default accuracy
-    of the 8-path maps over all frames."""
+    beside them a one-pair batch) with every frame copied from pinned host
+    memory and its map copied back (timed), 4-path vs 8-path; then P1/P2
+    fitted by 50 Adam steps on the soft-argmin L1 loss (FP32 BT volume, adjoint
+    kernels) and the refit vs default accuracy of the 8-path maps over all
+    frames."""
     import torch
 
     from thundervision_b200 import video
@@ -846,7 +847,7 @@ def measure_video(ctx, dev, n_frames=300, refit_steps=50):
             ms = loop.run(host, out_host)
             maps = [o.to(dev) for o in out_host]
             res[key] = {"engine": engine, "fps": n_frames / (ms / 1000.0), "ms_per_frame": ms / n_frames,
-                        **({"tiles": loop.tiles} if loop.tiles else {}), **mean_acc(maps)}
+                        **({"tiles": {"order": loop.tiles["order"]}} if loop.tiles else {}), **mean_acc(maps)}
             loop.close()
     # P1/P2 refit through the adjoint, then the 8-path maps with both settings
     fit_frames = [(l, r, gt.to(torch.int64), occ) for (l, r, gt, occ) in frames[:refit_steps]]

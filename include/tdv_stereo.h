@@ -166,22 +166,26 @@ tdv_status tdv_fast_wta_filtered(tdv_ctx* ctx, const tdv_image* left, const tdv_
  * the role of SemiGlobalLabDevRun (tdvision/semiglobal_lab.cu:232-282) with
  * the reference's cost and recurrence.  Integer-domain inputs (u8, scale 1,
  * P1/P2 multiples of 1/2, P2_CONST, D <= 256; any semantics and table whose
- * 16-bit ranges hold) take the fused 16-bit path; anything else runs
- * tdv_cost + tdv_sgm on context scratch. */
+ * 16-bit ranges hold) take the fused path: every direction at once, one byte
+ * per cell and direction, for P1/P2 up to 127.5 and where the allocator has
+ * those volumes (at most 10 GB); else passes that accumulate into a 16-bit
+ * volume.  Anything else runs tdv_cost + tdv_sgm on context scratch. */
 tdv_status tdv_stereo_sgm(tdv_ctx* ctx, const tdv_image* left, const tdv_image* right,
                           int32_t max_disp, const tdv_sgm_params* params, tdv_disparity* out,
                           tdv_stream stream);
 
 /* tdv_stereo_sgm's fused path over n frame pairs of one size (left[i],
  * right[i] -> out[i]), for a frame stream: the frames alternate between two
- * lanes, each with its own planes, aggregation volumes and streams, so that
- * one frame's DRAM-bound passes run while the other lane's last pass (WTA and
- * left-right check, bound by its instruction stream) finishes.  The call
+ * lanes, each with its own planes, volumes and streams, so that one lane's
+ * line kernel (bound by its instruction stream) can run beside the other
+ * lane's sum.  Under the reference CPU recurrence that gains nothing over
+ * single calls, under the others about 5 % at 1920x1080, D = 256.  The call
  * orders everything after the work already queued on `stream` and before the
  * work queued on it afterwards; the outputs must not overlap one another.
  * Maps are identical to n tdv_stereo_sgm calls.  Inputs outside the fused
- * path return TDV_ERR_UNSUPPORTED.  The second lane's scratch (about as much
- * as the first's) is allocated on the first call with n > 1.  No reference
+ * path return TDV_ERR_UNSUPPORTED.  The second lane's scratch (as much as
+ * the first's: 6.4 GB at 1920x1080, D = 256) is allocated on the first call
+ * with n > 1.  No reference
  * counterpart: the reference matches one pair per pipeline update
  * (tdvision/devstereomatcher.cpp:36-48). */
 tdv_status tdv_stereo_sgm_frames(tdv_ctx* ctx, int32_t n, const tdv_image* left, const tdv_image* right,
@@ -435,15 +439,22 @@ tdv_status tdv_ctx_set_allocator(tdv_ctx* ctx, tdv_alloc_fn alloc, tdv_free_fn r
                                  void* user);
 /* Pre-sizes the scratch of tdv_stereo_sgm (the fused path: planes, both
  * 16-bit aggregation volumes, the row scratch, and where the allocator has
- * room the eight byte volumes of the directions stored apart) for pairs up to
- * W x H x D, so later calls of it do not allocate.  The general path sizes its
- * own scratch on first use, once per size: tdv_sgm (up to eight volumes of W x H x D
- * floats while they fit 10 GB, four or two of them or none where the allocator
- * refuses; the aggregation volume, the path schedule, the deferred costs of
- * repeated walks), tdv_dp_scanline (W x H x D choice bytes), the filter-then-cost
- * case of tdv_cost_filtered (both filtered images).  A caller that must not
- * allocate later makes one call of each kind first, or passes its own
- * volumes. */
+ * room and they stay within 10 GB the eight byte volumes of the directions
+ * stored apart) for pairs up to W x H x D, so later calls of it do not
+ * allocate.  The general path sizes its own scratch on first use, once per
+ * size: tdv_sgm (up to eight volumes of W x H x D floats while they fit 10 GB,
+ * four or two of them or none where the allocator refuses; the aggregation
+ * volume, the path schedule, the deferred costs of repeated walks),
+ * tdv_dp_scanline (W x H x D choice bytes), the filter-then-cost case of
+ * tdv_cost_filtered (both filtered images).  A caller that must not allocate
+ * later makes one call of each kind first, or passes its own volumes.
+ *
+ * What only speeds a call up (the byte volumes, tdv_sgm's side-by-side
+ * volumes) is given back when necessary scratch does not fit, unless a
+ * captured call uses it; a refused request is made again after 64 calls.  A
+ * captured tdv_sgm call without a volume of its own takes tdv_sgm's volumes
+ * over for its replays; one into the caller's own volume runs its passes in
+ * sequence there and shares no scratch volume with any other call. */
 tdv_status tdv_ctx_reserve(tdv_ctx* ctx, int32_t width, int32_t height, int32_t max_disp);
 const char* tdv_last_error_string(const tdv_ctx* ctx);
 /* Synchronises `stream` and returns the error status kernels of this

@@ -8,8 +8,8 @@ per pipeline update, tdvision/devstereomatcher.cpp:36-48).
   for the per-frame noise, so 300 full-HD frames take seconds instead of
   minutes of host time.
 * ``VideoLoop`` -- frames from pinned host memory through one CUDA graph
-  replay per frame (a persistent batch launch, or the per-frame fused kernels
-  of tdv_stereo_sgm with their two concurrent chains): the copy of frame t+1
+  replay per frame (the launches of a one-pair batch, or the fused kernels of
+  tdv_stereo_sgm): the copy of frame t+1
   runs on a copy stream while frame t is aggregated (two input buffer sets),
   and each frame's disparity map is copied back to pinned host memory.
 * ``refit_penalties`` -- fits P1, P2 by gradient steps on the soft-argmin L1
@@ -87,9 +87,9 @@ class VideoLoop:
     """Double-buffered frame loop, one CUDA graph replay per frame.
 
     ``engine="launches"`` (default): each frame is the per-frame fused
-    kernels of tdv_stereo_sgm (two concurrent pass chains), captured into one
-    CUDA graph per buffer set.  ``engine="persistent"``: each frame is one
-    persistent batch launch (tdv_batch_graph_launch, tiles autotuned once).
+    kernels of tdv_stereo_sgm, captured into one CUDA graph per buffer set.
+    ``engine="persistent"``: each frame is a one-pair batch run
+    (tdv_batch_graph_launch, autotuned once).
     ``paths`` 4 or 8; P1/P2 must be multiples of 1/2 (the integer-domain
     fused path).  ``semantics`` / ``table`` (launches engine): "standard" /
     "full", or "ref_cpu" / "ref" for the reference's own CPU recurrence over
@@ -97,10 +97,9 @@ class VideoLoop:
     kernels also run; the persistent engine takes the standard ones only.
 
     ``overlap=True`` (launches engine): each buffer set has its own private
-    context (its own aggregation volumes) and its own compute stream, so
-    frame t+1's passes can run while frame t finishes: the last horizontal
-    pass, bound by its instruction stream, overlaps the next frame's
-    DRAM-bound passes.  Maps are the same as with one context.
+    context (its own volumes) and its own compute stream, so frame t+1's line
+    kernel (bound by its instruction stream) can run beside frame t's sum.
+    Maps are the same as with one context.
     """
 
     def __init__(self, ctx, W, H, D, p1, p2, paths=8, lr=1, graph=True, autotune=True, device="cuda",

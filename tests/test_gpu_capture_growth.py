@@ -3,6 +3,8 @@ graph writes is neither freed nor handed back when a call with other paths,
 another disparity range of the same class, another recurrence or a larger
 volume of its own comes after it.  What the allocator was asked to release is
 checked before the graph is replayed (and kept, filled with ones)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -105,3 +107,52 @@ def test_own_volume_then_a_larger_range():
     _replay_after(lambda c: None, lambda c: c.sgm(small, 0.1, 0.5, aggreg=s_small),
                   [lambda c: c.sgm(large, 0.1, 0.5, aggreg=s_large)], none_released=False)
     plain.close()
+
+
+def _cudart():
+    with open("/proc/self/maps") as f:
+        paths = {ln.split()[-1] for ln in f if "libcudart.so" in ln}
+    return ctypes.CDLL(sorted(paths)[0])
+
+
+def test_capture_behind_a_queued_call():
+    """A capture begun while the warm-up call is still queued, as a C caller may
+    (torch's own capture waits first): the graph gets the side-by-side volumes
+    all the same, so the next direct call allocates its own."""
+    f = [p.float() / 255 for p in _pair()]
+    c, live, _ = _context()
+    plain = api.Context(0)
+    rt = _cudart()
+    graph, gexec = ctypes.c_void_p(), ctypes.c_void_p()
+    try:
+        cost = plain.cost(*f, 32)
+        own = torch.empty_like(cost)
+        want = plain.sgm(cost, 0.1, 0.5)["disp"].to(torch.int32)
+        c.sgm(cost, 0.1, 0.5)
+        s = torch.cuda.Stream()
+        st = ctypes.c_void_p(s.cuda_stream)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s):
+            c.sgm(cost, 0.1, 0.5)  # leaves a cached output block to the captured call
+            torch.cuda._sleep(400_000_000)
+            c.sgm(cost, 0.1, 0.5)
+            assert not s.query()
+            assert rt.cudaStreamBeginCapture(st, 0) == 0
+            out = c.sgm(cost, 0.1, 0.5)["disp"]
+            assert rt.cudaStreamEndCapture(st, ctypes.byref(graph)) == 0
+            assert rt.cudaGraphInstantiate(ctypes.byref(gexec), graph, ctypes.c_ulonglong(0)) == 0
+            n = len(live)
+            direct = c.sgm(cost, 0.1, 0.5, aggreg=own)["disp"]
+            assert len(live) == n + 1
+            assert rt.cudaGraphLaunch(gexec, st) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out.to(torch.int32), want)
+        assert torch.equal(direct.to(torch.int32), want)
+    finally:
+        torch.cuda.synchronize()
+        if gexec:
+            rt.cudaGraphExecDestroy(gexec)
+        if graph:
+            rt.cudaGraphDestroy(graph)
+        c.close()
+        plain.close()

@@ -121,16 +121,16 @@ bool grow_optional(tdv_ctx* ctx, tdv_ctx::OptBuf& b, size_t bytes) {
     return true;
 }
 
-// Whether an event recorded outside any capture has passed, asked while a
-// stream of this thread may be capturing.
-bool idle(cudaEvent_t ev) {
+// Waits on the host for an event recorded outside any capture, while a stream of
+// this thread may be capturing; false if that fails.
+bool passed(cudaEvent_t ev) {
     if (!ev) return true;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    const bool done = cudaEventQuery(ev) == cudaSuccess;
+    const bool done = cudaEventSynchronize(ev) == cudaSuccess;
     if (!done) cudaGetLastError();
     cudaThreadExchangeStreamCaptureMode(&mode);
     return done;
@@ -271,9 +271,9 @@ tdv_status ensure_schedule(tdv_ctx* ctx, int W, int H, int table, int paths, cud
 //
 // Direct calls share sgm_part: each waits for the one before it, on whatever
 // stream that ran.  A capturing call allocates nothing and its replays run
-// beside direct calls, so it takes sgm_part over for good (idle, and larger than
-// what earlier captures took) as sgm_graph, and the next direct call allocates
-// again.  Replays that share sgm_graph also share the context's aggregation
+// beside direct calls, so it takes sgm_part over for good (once the direct calls
+// queued on it are through, and if it is larger than what earlier captures took)
+// as sgm_graph, and the next direct call allocates again.  Replays that share sgm_graph also share the context's aggregation
 // volume; a capture into the caller's own volume shares nothing with any other
 // call, and stays so: in sequence.
 int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool own, cudaStream_t st, tdv_ctx::OptBuf** part) {
@@ -286,7 +286,7 @@ int side_by_side(tdv_ctx* ctx, int W, int H, int D, int sem, bool own, cudaStrea
     if (captured && own) return 0;
     const int most = fit ? all : std::min(all, 4);
     if (captured && ctx->sgm_graph.bytes < most * vol && ctx->sgm_part.bytes > ctx->sgm_graph.bytes &&
-        ctx->retired_bytes + ctx->sgm_graph.bytes <= kMaxOptional && idle(ctx->sgm_done)) {
+        ctx->retired_bytes + ctx->sgm_graph.bytes <= kMaxOptional && passed(ctx->sgm_done)) {
         if (ctx->sgm_graph.ptr) {
             ctx->retired.push_back(ctx->sgm_graph);
             ctx->retired_bytes += ctx->sgm_graph.bytes;

@@ -55,3 +55,13 @@ def test_wide(ctx, orc, kind, radius, D):
         C = ctx.cost(L, R, D, kind="ssd", radius=radius)
         assert torch.equal(ctx.fast_wta(L, R, D, radius=radius)["disp"].view(torch.int16),
                            ctx.wta(C)["disp"].view(torch.int16))
+
+
+@pytest.mark.parametrize("kind,radius,W,H,D", [
+    # either side of the tile counts from which tiles are 8 rows high
+    ("bt", 0, 641, 217, 16), ("bt", 0, 641, 222, 16), ("bt", 0, 641, 222, 17),
+    ("ncc", 4, 641, 433, 8), ("ncc", 4, 641, 438, 8), ("ncc", 2, 641, 438, 9), ("ncc", 4, 1283, 459, 16),
+    # the 3x3 of 16 lanes: two rows an item, then one
+    ("ncc", 1, 641, 217, 20), ("ncc", 1, 641, 222, 20), ("ncc", 1, 1283, 565, 31), ("ncc", 2, 1283, 565, 31)])
+def test_tile_counts(ctx, orc, kind, radius, W, H, D):
+    _check(ctx, orc, kind, radius, W, H, D)

@@ -657,6 +657,9 @@ __global__ void __launch_bounds__(kThreads, 3) fastwta_band_kernel(ImgArg L, Img
     }
 }
 
+// How many tiles of 8 rows an image has.
+long long tall_tiles(int W, int H) { return (long long)((W + kTX - 1) / kTX) * ((H + 7) / 8); }
+
 // Tile height.  8 rows share a window's halo, its filter and its window sums
 // better, 4 spread a small image over the chip (NCC 9x9, D = 64: 0.603 / 0.620
 // ms at 1920x1080, 0.120 / 0.110 at 640x480; BT 0.125 / 0.132 and 0.029 /
@@ -669,7 +672,11 @@ __global__ void __launch_bounds__(kThreads, 3) fastwta_band_kernel(ImgArg L, Img
 //   * for SSD up to D = 16 always: a work item is then 32 or 64 pixels of two
 //     rows, and 4 rows leave half the block's warps without one (7x7 filtered,
 //     640x480, D = 8: 24 us against 34);
-//   * not for the 9x9 NCC up to D = 31 (1280x720, D = 16: 118 us against 112).
+//   * for BT up to D = 16 from two rounds on (D = 8, 4 / 8 rows: 160x120 4.2 /
+//     6.3 us, 436x804 12.4 / 10.4, 1003x701 18.6 / 16.5);
+//   * for NCC up to D = 8 from four rounds on (9x9, 1003x701, D = 8: 69 / 60),
+//     up to D = 16 from eight (5x5, 800x450, D = 16: 27.0 / 28.8);
+//   * not for the 9x9 NCC of D = 17 to 31 (1280x720, D = 20: 162 us against 170).
 // 2 rows where a block of 4 takes an SM for itself (NCC 3x3, D = 1900, 640x128:
 // 0.73 ms against 0.79 with 4); FastWTA keeps 4 there (it measured slower with
 // 2: 7x7, D = 1800, 0.89 ms against 0.75).
@@ -680,11 +687,11 @@ int band_bytes(const Geom& g) {
 }
 template <int KIND, int R, int HP, bool FILT>
 int tile_rows(int W, int H, const Geom& g) {
-    const long long tiles = (long long)((W + kTX - 1) / kTX) * ((H + 7) / 8);
+    const long long tiles = tall_tiles(W, H);
     long long tall = 1480;
     if (KIND == TDV_COST_BT && g.D > 100) tall = 2960;
-    if (KIND != TDV_COST_NCC && g.D <= 16) tall = 0;
-    const bool never = KIND == TDV_COST_NCC && R == 4 && !FILT && g.Dw == 16;
+    if (g.D <= 16) tall = KIND == TDV_COST_SSD ? 0 : (KIND == TDV_COST_BT ? 300 : (g.D <= 8 ? 600 : 1200));
+    const bool never = KIND == TDV_COST_NCC && R == 4 && !FILT && g.Dw == 16 && g.D > 16;
     if (!never && tiles >= tall && band_bytes<KIND, R, HP, FILT, 8>(g) <= kThreeBlocks) return 8;
     return KIND == TDV_COST_BT || band_bytes<KIND, R, HP, FILT, 4>(g) <= kTwoBlocks ? 4 : 2;
 }
@@ -739,10 +746,16 @@ cudaError_t launch_nr(const ImgArg& L, const ImgArg& Rim, const VolArg& out, con
 template <int KIND, int R, int P, bool FILT, int TY>
 cudaError_t launch_ty(const ImgArg& L, const ImgArg& Rim, const VolArg& out, const Geom& g, float* fl_out,
                       cudaStream_t st) {
-    // NCC of narrow lane groups: one row per item, so that every warp has one
-    // (9x9, 160x120, D = 16: 14 us, with two rows 19)
+    // NCC of narrow lane groups: one row per item where two would leave a warp
+    // without one (9x9, 160x120, D = 16: 14 us, with two rows 19; where every
+    // warp has one, two rows share the window sums: 436x804, D = 20, 70 against
+    // 78), and for the 3x3 of 16 lanes, whose sums are short (1920x1080, D = 16:
+    // 90 against 100; 640x480, D = 31: 29.0 against 30.7), from two rounds of
+    // tiles over 148 SMs on (320x240, D = 20, filtered: 16.5 against 14.5).
     if constexpr (KIND == TDV_COST_NCC && TY > 2)
-        if (g.Dw < 32) return launch_nr<KIND, R, P, FILT, TY, 1>(L, Rim, out, g, fl_out, st);
+        if (TY / 2 * (kTX / (P * g.G)) * ((g.D + g.Dw - 1) / g.Dw) < kWarps ||
+            (R == 1 && g.Dw == 16 && tall_tiles(out.W, out.H) >= 300))
+            return launch_nr<KIND, R, P, FILT, TY, 1>(L, Rim, out, g, fl_out, st);
     return launch_nr<KIND, R, P, FILT, TY, 2>(L, Rim, out, g, fl_out, st);
 }
 
